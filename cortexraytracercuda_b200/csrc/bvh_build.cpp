@@ -551,4 +551,30 @@ void collapse_leaves(BvhOutput& t, int max_leaf) {
     t.max_leaf_seen = max_leaf_seen;
 }
 
+// Renumbers the leaf slots in depth-first order, left child first, so that the leaves of one node are
+// consecutive (the walk tests them as one range) and neighbouring leaves share cache lines.
+void order_leaves(BvhOutput& t) {
+    std::vector<uint32_t> order;
+    order.reserve(t.order.size());
+    std::vector<std::pair<uint32_t, int>> work;   // (node, side) still to take
+    if (t.num_nodes) work = {{0u, 1}, {0u, 0}};
+    while (!work.empty()) {
+        const auto [node, side] = work.back();
+        work.pop_back();
+        float* at = &t.nodes[16 * (size_t)node + 12 + side];
+        int32_t c;
+        std::memcpy(&c, at, 4);
+        if (c >= 0) {
+            work.push_back({(uint32_t)c, 1});
+            work.push_back({(uint32_t)c, 0});
+            continue;
+        }
+        const uint32_t first = (uint32_t)~c >> LEAF_COUNT_BITS, cnt = (uint32_t)~c & MAX_LEAF;
+        const int32_t enc = (int32_t)~(((uint32_t)order.size() << LEAF_COUNT_BITS) | cnt);
+        std::memcpy(at, &enc, 4);
+        for (uint32_t k = 0; k < cnt; ++k) order.push_back(t.order[first + k]);
+    }
+    t.order.swap(order);
+}
+
 }  // namespace rtc

@@ -41,6 +41,10 @@ bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, co
 // updates num_nodes, max_depth and max_leaf_seen.  For one-primitive-per-leaf trees.
 void collapse_leaves(BvhOutput& tree, int max_leaf);
 
+// Renumbers the leaf slots depth-first, left child first, as build_bvh lays them out: two leaves of one
+// node are then consecutive.  For the device builds' trees.
+void order_leaves(BvhOutput& tree);
+
 // BVH built on CUDA device `device` (bvh_device.cu) over Morton-sorted primitives, one primitive per
 // leaf, no 8-wide nodes: PLOC clustering (BVH_DEVICE_PLOC) or the linear BVH (BVH_DEVICE_LBVH).
 // BVH_DEVICE_TOO_DEEP and BVH_DEVICE_UNSUPPORTED leave the SAH build as the way out.

@@ -527,6 +527,7 @@ int build_bvh_device(const BvhInput& in, int device, BvhDeviceMethod method, Bvh
         // one primitive per leaf so far: with RTC_DEVICE_LEAF_MAX > 1, merge small subtrees into leaves of
         // up to that many where the SAH cost favours it, as the host build's leaves are
         if (RTC_DEVICE_LEAF_MAX > 1) collapse_leaves(out, RTC_DEVICE_LEAF_MAX);
+        order_leaves(out);
         if (out.max_depth + 2 > (uint32_t)TRAVERSAL_STACK) {
             what = "device BVH too deep for the traversal stack";
             rc = BVH_DEVICE_TOO_DEEP;

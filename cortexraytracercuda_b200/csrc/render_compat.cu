@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128) rtc_trace_closest(DevScene S, const float
     float t;
     uint32_t item, status = 0;
     TraceStats st{0, 0};
-    bool h = closest_hit<false, WIDE>(S, o, d, R[3], R[7], depth == max_depth, t, item, st, status);
+    bool h = closest_hit<false, WIDE ? WALK_WIDE : WALK_BINARY>(S, o, d, R[3], R[7], depth == max_depth, t, item, st, status);
     if (prim) prim[k] = h ? item_gid(S, item) : -1;
     if (tout) tout[k] = h ? t : INFINITY;
     if (status) atomicOr(status_word, status);

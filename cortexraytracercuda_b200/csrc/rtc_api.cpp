@@ -269,6 +269,35 @@ void rtc_view_env_sampling(DevScene& S, const rtc_render_params* p) {
 }
 DevParams rtc_dev_params(const rtc_render_params* p);
 
+// Checks a binary tree's links and leaf ranges against its node and item counts, and that two leaves of
+// one node are consecutive (left first; an empty leaf may point anywhere), then writes each leaf's first
+// item word where the leaf's items are consecutive words (rtc_dev.h).  `items` null: an xprim tree, whose
+// items are 0, 1, 2, ... and whose nodes carry no words.
+static bool check_tree(BvhOutput& t, const uint32_t* items, uint32_t num_items) {
+    for (uint32_t n = 0; n < t.num_nodes; ++n) {
+        float* f = &t.nodes[16 * (size_t)n];
+        int32_t link[2];
+        std::memcpy(link, f + 12, sizeof link);
+        uint32_t word[2] = {0xffffffffu, 0xffffffffu}, first[2] = {0, 0}, cnt[2] = {0, 0};
+        for (int side = 0; side < 2; ++side) {
+            if (link[side] >= 0) {
+                if ((uint32_t)link[side] >= t.num_nodes) return false;
+                continue;
+            }
+            first[side] = (uint32_t)~link[side] >> LEAF_COUNT_BITS;
+            cnt[side] = (uint32_t)~link[side] & MAX_LEAF;
+            if (first[side] + cnt[side] > num_items) return false;
+            if (!items || cnt[side] == 0) continue;
+            word[side] = items[first[side]];
+            for (uint32_t k = 1; k < cnt[side]; ++k)
+                if (items[first[side] + k] != word[side] + k) word[side] = 0xffffffffu;
+        }
+        if (link[0] < 0 && link[1] < 0 && cnt[0] && cnt[1] && first[1] != first[0] + cnt[0]) return false;
+        std::memcpy(f + 14, word, sizeof word);
+    }
+    return true;
+}
+
 rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t bvh_builder, int device) {
     if (!d) return fail(RTC_ERR_INVALID_ARGUMENT, "null argument");
     if (bvh_builder != RTC_BVH_SAH && bvh_builder != RTC_BVH_DEVICE && bvh_builder != RTC_BVH_DEVICE_LBVH)
@@ -555,7 +584,7 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     }
 
     // ---- per-kind arrays in leaf order ---------------------------------------------------------
-    std::vector<uint32_t> items(bvh.order.size()), xitems(xbvh.order.size());
+    std::vector<uint32_t> items(bvh.order.size());
     std::vector<float4> sph, tri, tri_n, tri_vn, tri_uv, quad, light(6 * (size_t)nlights), rect, xf;
     // per-vertex texture coordinates: when any mesh has them, every triangle gets a uv record (zeros
     // for meshes without)
@@ -679,9 +708,16 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
             xprim.push_back(make_int4(pr.xf, pr.inner, (int)inner, (int)gid));
         } break;
         }
-        (xk ? xitems[k - bvh.order.size()] : items[k]) = ((uint32_t)pr.kind << ITEM_KIND_SHIFT) | typed;
+        if (!xk) items[k] = ((uint32_t)pr.kind << ITEM_KIND_SHIFT) | typed;   // an xprim's leaf item is its index
     }
     for (uint32_t i = 0; i < d->num_transforms; ++i) put_transform(d->transforms[i], xf);
+    // The walks read links, leaf ranges and item words without checking them, so they are checked here.
+    const uint32_t kind_count[4] = {(uint32_t)sph.size(), (uint32_t)(quad.size() / 5), (uint32_t)tri_n.size(), nlights};
+    for (uint32_t it : items)
+        if ((it >> ITEM_KIND_SHIFT) > ITEM_LIGHT || (it & ITEM_INDEX_MASK) >= kind_count[it >> ITEM_KIND_SHIFT])
+            return bad("inconsistent leaf items");
+    if (!check_tree(bvh, items.data(), (uint32_t)items.size()) || !check_tree(xbvh, nullptr, (uint32_t)xprim.size()))
+        return bad("inconsistent BVH");
     // the 8-wide nodes' leaf items: the same item words, regrouped per wide node
     std::vector<uint32_t> items8(bvh.items8.size());
     for (size_t k = 0; k < items8.size(); ++k) items8[k] = items[bvh.items8[k]];
@@ -722,7 +758,6 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     size_t o_xf = add_chunk(xf.data(), xf.size() * 16);
     size_t o_rect = add_chunk(rect.data(), rect.size() * 16);
     size_t o_xnodes = add_chunk(xbvh.nodes.data(), xbvh.nodes.size() * sizeof(float));
-    size_t o_xitems = add_chunk(xitems.data(), xitems.size() * 4);
     size_t env_bytes = d->background.kind == RTC_BG_ENV_MAP
                            ? (size_t)d->background.env_width * d->background.env_height * 3 * sizeof(float) : 0;
     size_t o_env = add_chunk(env_bytes ? d->background.env_rgb : nullptr, env_bytes);
@@ -792,9 +827,7 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     D.num_xf = d->num_transforms;
     D.num_rect = (uint32_t)(rect.size() / 2);
     D.xnodes = xbvh.num_nodes ? (const float4*)off(o_xnodes) : nullptr;
-    D.xitems = xbvh.num_nodes ? (const uint32_t*)off(o_xitems) : nullptr;
     D.num_xnodes = xbvh.num_nodes;
-    D.num_xitems = (uint32_t)xitems.size();
     D.num_nodes = bvh.num_nodes;
     D.num_nodes8 = bvh.num_nodes8;
     D.num_items = (uint32_t)items.size();
@@ -839,7 +872,7 @@ DevScene rtc_rebase_scene(const HostScene& H, uint8_t* base) {
     rb(D.sph); rb(D.sph_aux); rb(D.tri); rb(D.tri_n); rb(D.tri_vn); rb(D.quad);
     rb(D.light); rb(D.mat_i); rb(D.mat_f); rb(D.tex_i); rb(D.tex_f); rb(D.images); rb(D.image_bytes);
     rb(D.xprim); rb(D.xf); rb(D.rect);
-    if (D.xnodes) { rb(D.xnodes); rb(D.xitems); }
+    if (D.xnodes) rb(D.xnodes);
     if (D.bg.env) rb(D.bg.env);
     if (D.bg.cdf) rb(D.bg.cdf);
     if (D.tri_uv) rb(D.tri_uv);

@@ -4,8 +4,11 @@
 //
 //   nodes      BVH2, 4 x float4 = 64 B per node:
 //                n0 = (L.lo.x, L.hi.x, L.lo.y, L.hi.y)   n1 = (R.lo.x, R.hi.x, R.lo.y, R.hi.y)
-//                n2 = (L.lo.z, L.hi.z, R.lo.z, R.hi.z)   n3 = (child L, child R, -, -) as int bits
-//              child >= 0: inner node index; child < 0: leaf, ~child = (first_item << 5) | count.
+//                n2 = (L.lo.z, L.hi.z, R.lo.z, R.hi.z)   n3 = (child L, child R, word L, word R) as int bits
+//              child >= 0: inner node index; child < 0: leaf, ~child = (first_item << 5) | count, and its
+//              word is the item word of its first item when the leaf's items are consecutive words
+//              (0xffffffff otherwise, and for inner children).  Two leaves of one node are consecutive in
+//              `items`, the left one first.
 //   nodes8     the same tree collapsed to 8-wide nodes with quantised child boxes, 5 x float4 = 80 B:
 //                (p.xyz, header)  header = (e.x+127) | (e.y+127) << 8 | (e.z+127) << 16 | valid << 24
 //                (child base, item base, link bytes of slots 0-3, link bytes of slots 4-7) as int bits
@@ -21,7 +24,8 @@
 //   items      uint32 per leaf entry, leaf order: (kind << 29) | index into that kind's array.
 //   xprim      int4 per transformed primitive or box face (leaf order): (transform or -1, inner kind,
 //              inner index, global id).  The inner record sits in the sph / quad / tri / rect array.
-//              Xprims have their own BVH2 (`xnodes`, leaves into `xitems`), walked after the main one.
+//              Xprims have their own BVH2 (`xnodes`), walked after the main one; a leaf's items are the
+//              xprims themselves.
 //   xf         8 x float4 per transform: (translate.xyz, flags) (scale.xyz, -) (inverse rotation columns
 //              0..2, xyz) (forward rotation columns 0..2, xyz), the glm matrices of rt::rotate
 //   rect       2 x float4 per box face: (a0, a1, b0, b1) (k, axis, flip, material); axis 0 = xy_rect
@@ -131,7 +135,6 @@ struct DevScene {
     const float4* xf;
     const float4* rect;
     const float4* xnodes;      // BVH2 over the xprims (null when there are none)
-    const uint32_t* xitems;
     uint32_t num_nodes;
     uint32_t num_nodes8;
     uint32_t num_items;
@@ -140,7 +143,7 @@ struct DevScene {
     uint32_t num_textures;
     uint32_t num_images;
     uint32_t num_sph, num_tri, num_quad;
-    uint32_t num_xprim, num_xf, num_rect, num_xnodes, num_xitems;
+    uint32_t num_xprim, num_xf, num_rect, num_xnodes;
     DevCamera cam;
     DevBackground bg;
 };

@@ -347,82 +347,85 @@ __device__ __forceinline__ bool rect_t(float4 r0, float4 r1, V3 o, V3 d, float t
     return !(a < r0.x || a > r0.y || b < r0.z || b > r0.w);
 }
 
-// Tests every item of one leaf against [tmin, best_t].  EXACT: clean mode's double-precision sphere test.
-// A leaf of the xprim BVH: transformed primitives and box faces, each tested on its object-space ray.
+// The object-space ray of the transform used last: the faces of a box and the triangles of a transformed
+// mesh share one transform, and their leaves follow each other in the walk, so the ray (three or six
+// divisions and two matrix products) is made once per change of transform, not once per primitive.
+struct XformRay {
+    int32_t xf;   // -1: the world ray
+    V3 o, d;
+};
+
+// A leaf range of the xprim BVH, xprims [first, first + cnt) (leaf order is xprim order: item k of the list
+// is xprim k): transformed primitives and box faces, each tested on its object-space ray.  EXACT: clean
+// mode's double-precision sphere test.  Links and indices were checked when the scene was created.
 template <bool EXACT>
-__device__ __forceinline__ void test_leaf_xprims(const DevScene& S, int32_t child, V3 o, V3 d, float tmin,
-                                                 float& best_t, uint32_t& best_item, TraceStats& st,
-                                                 uint32_t& status) {
-    const uint32_t enc = (uint32_t)(~child);
-    const uint32_t first = enc >> LEAF_COUNT_BITS, cnt = enc & MAX_LEAF;
-    if (first + cnt > S.num_xitems) { status |= STATUS_BAD_ITEM; return; }
-    for (uint32_t k = 0; k < cnt; ++k) {
-        const uint32_t it = ld_scene(S.xitems + first + k);
-        const uint32_t idx = it & ITEM_INDEX_MASK;
+__device__ __forceinline__ void test_xprims(const DevScene& S, uint32_t first, uint32_t cnt, V3 o, V3 d, XformRay& xr,
+                                            float tmin, float& best_t, uint32_t& best_item, TraceStats& st,
+                                            uint32_t& status) {
+    for (uint32_t idx = first; idx < first + cnt; ++idx) {
         st.prims++;
-        if ((it >> ITEM_KIND_SHIFT) != ITEM_XPRIM || idx >= S.num_xprim) { status |= STATUS_BAD_ITEM; continue; }
         const int4 x = __ldg(S.xprim + idx);
-        V3 ro = o, rd = d;
-        if (x.x >= 0) {
-            if ((uint32_t)x.x >= S.num_xf) { status |= STATUS_BAD_ITEM; continue; }
-            xf_to_object(S, x.x, ro, rd);
+        if (x.x != xr.xf) {
+            xr.xf = x.x;
+            xr.o = o;
+            xr.d = d;
+            if (x.x >= 0) xf_to_object(S, x.x, xr.o, xr.d);
         }
         const uint32_t in = (uint32_t)x.z;
         float t;
         bool h = false;
         switch (x.y) {
         case ITEM_SPHERE: {
-            if (in >= S.num_sph) { status |= STATUS_BAD_ITEM; break; }
             const float4 sp = ld_scene(S.sph + in);
-            h = EXACT ? sphere_t_exact(sp, ro, rd, tmin, best_t, t) : sphere_t(sp, ro, rd, tmin, best_t, t);
+            h = EXACT ? sphere_t_exact(sp, xr.o, xr.d, tmin, best_t, t) : sphere_t(sp, xr.o, xr.d, tmin, best_t, t);
         } break;
         case ITEM_QUAD: {
-            if (in >= S.num_quad) { status |= STATUS_BAD_ITEM; break; }
             const float4* q = S.quad + 5 * (size_t)in;
             float a, b;
-            h = planar_t(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3), __ldg(q + 4), ro, rd, tmin, best_t, false, t, a, b);
+            h = planar_t(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3), __ldg(q + 4), xr.o, xr.d, tmin, best_t, false, t, a, b);
         } break;
         case ITEM_TRI: {
-            if (in >= S.num_tri) { status |= STATUS_BAD_ITEM; break; }
             const float4* p = S.tri + 3 * (size_t)in;
             float bu, bv;
-            h = tri_t(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), ro, rd, tmin, best_t, t, bu, bv);
+            h = tri_t(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), xr.o, xr.d, tmin, best_t, t, bu, bv);
         } break;
         case XPRIM_RECT: {
-            if (in >= S.num_rect) { status |= STATUS_BAD_ITEM; break; }
             float a, b;
-            h = rect_t(__ldg(S.rect + 2 * (size_t)in), __ldg(S.rect + 2 * (size_t)in + 1), ro, rd, tmin, best_t, t, a, b);
+            h = rect_t(__ldg(S.rect + 2 * (size_t)in), __ldg(S.rect + 2 * (size_t)in + 1), xr.o, xr.d, tmin, best_t, t, a, b);
         } break;
         default: status |= STATUS_BAD_ITEM; break;
         }
         if (h) {
             best_t = t;
-            best_item = it;
+            best_item = ((uint32_t)ITEM_XPRIM << ITEM_KIND_SHIFT) | idx;
         }
     }
 }
 
+// A leaf range's items not known to be consecutive item words (see test_items).
+constexpr uint32_t ITEMS_LISTED = 0xffffffffu;
+
 // Items [first, first + cnt) of an item list (`items`, or `items8` for the 8-wide nodes; both hold
-// num_items entries) against [tmin, best_t].
+// num_items entries) against [tmin, best_t].  `word` is the first item's word when the range's items are
+// consecutive words - one kind, indices in leaf order, which is how the primitives are packed - so that
+// the walk goes from the node straight to the primitive record; ITEMS_LISTED reads the list.  Words and
+// ranges were checked when the scene was created (rtc_api.cpp, check_tree), not per test.
 template <bool EXACT>
-__device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* items, uint32_t first, uint32_t cnt,
+__device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* items, uint32_t first, uint32_t cnt, uint32_t word,
                                            V3 o, V3 d, float tmin, float& best_t, uint32_t& best_item,
                                            bool hide_invisible, TraceStats& st, uint32_t& status) {
-    if (first + cnt > S.num_items) { status |= STATUS_BAD_ITEM; return; }
     for (uint32_t k = 0; k < cnt; ++k) {
-        uint32_t it = ld_scene(items + first + k);
+        const uint32_t it = word != ITEMS_LISTED ? word + k : ld_scene(items + first + k);
         uint32_t kind = it >> ITEM_KIND_SHIFT, idx = it & ITEM_INDEX_MASK;
         float t;
         st.prims++;
         switch (kind) {
         case ITEM_TRI: {
-            if (idx >= S.num_tri) { status |= STATUS_BAD_ITEM; break; }
             const float4* p = S.tri + 3 * (size_t)idx;
             float bu, bv;
             if (tri_t(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), o, d, tmin, best_t, t, bu, bv)) { best_t = t; best_item = it; }
         } break;
         case ITEM_SPHERE: {
-            if (idx >= S.num_sph) { status |= STATUS_BAD_ITEM; break; }
             const float4 sp = ld_scene(S.sph + idx);
             if (EXACT ? sphere_t_exact(sp, o, d, tmin, best_t, t) : sphere_t(sp, o, d, tmin, best_t, t)) {
                 best_t = t;
@@ -430,7 +433,6 @@ __device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* it
             }
         } break;
         case ITEM_QUAD: {
-            if (idx >= S.num_quad) { status |= STATUS_BAD_ITEM; break; }
             const float4* q = S.quad + 5 * (size_t)idx;
             float a, b;
             if (planar_t(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3), __ldg(q + 4), o, d, tmin, best_t, false, t, a, b)) {
@@ -439,7 +441,6 @@ __device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* it
             }
         } break;
         case ITEM_LIGHT: {
-            if (idx >= S.num_lights) { status |= STATUS_BAD_ITEM; break; }
             const float4* q = S.light + 6 * (size_t)idx;
             float a, b;
             const float4 q3 = __ldg(q + 3), q4 = __ldg(q + 4);
@@ -458,16 +459,6 @@ __device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* it
         default: status |= STATUS_BAD_ITEM; break;
         }
     }
-}
-
-// A binary leaf: child = ~((first << LEAF_COUNT_BITS) | count) over `items`.
-template <bool EXACT>
-__device__ __forceinline__ void test_leaf(const DevScene& S, int32_t child, V3 o, V3 d, float tmin, float& best_t,
-                                          uint32_t& best_item, bool hide_invisible, TraceStats& st,
-                                          uint32_t& status) {
-    const uint32_t enc = (uint32_t)(~child);
-    test_items<EXACT>(S, S.items, enc >> LEAF_COUNT_BITS, enc & MAX_LEAF, o, d, tmin, best_t, best_item,
-                      hide_invisible, st, status);
 }
 
 // Direction component for the slab tests' reciprocal.  The slab distance is fma(lo, 1/d, -o/d); with a
@@ -614,8 +605,10 @@ __device__ __forceinline__ bool closest_hit8(const DevScene& S, V3 o, V3 d, V3 i
             }
             visit = links.x + (int32_t)(lb & 7u);
         } else {
-            test_items<EXACT>(S, S.items8, (uint32_t)links.y + (lb & 31u), ((lb >> 5) & 3u) + 1u, o, d, tmin, best_t,
-                              best_item, hide_invisible, st, status);
+            const uint32_t first = (uint32_t)links.y + (lb & 31u), cnt = ((lb >> 5) & 3u) + 1u;
+            if (first + cnt > S.num_items) { status |= STATUS_BAD_ITEM; break; }
+            test_items<EXACT>(S, S.items8, first, cnt, ITEMS_LISTED, o, d, tmin, best_t, best_item, hide_invisible, st,
+                              status);
         }
     }
     t_out = best_t;
@@ -623,7 +616,29 @@ __device__ __forceinline__ bool closest_hit8(const DevScene& S, V3 o, V3 d, V3 i
     return best_item != 0xffffffffu;
 }
 
-// The xprim BVH (binary, `xnodes` / `xitems`) against [tmin, best_t]: updates best_t / best_item and
+// One step of a binary walk after a node's slab test: the hit leaves as one range of items.  A leaf child
+// is tested before any inner child is walked, the left one first, and the leaves of one node are
+// consecutive in the item list (the builders number them so; checked with the scene), so both together
+// are one range: their lanes run one test loop per visit instead of one per side.  Returns false when
+// neither child is a hit leaf; clears hl / hr of the leaves it takes.
+__device__ __forceinline__ bool hit_leaves(int32_t cl, int32_t cr, uint32_t wl, uint32_t wr, bool& hl, bool& hr,
+                                           uint32_t& first, uint32_t& cnt, uint32_t& word) {
+    const bool lf = hl && cl < 0, rf = hr && cr < 0;
+    if (!lf && !rf) return false;
+    const uint32_t enc = (uint32_t)~(lf ? cl : cr);
+    first = enc >> LEAF_COUNT_BITS;
+    cnt = enc & MAX_LEAF;
+    word = lf ? wl : wr;
+    if (lf && rf) {
+        if (wr != word + cnt) word = ITEMS_LISTED;
+        cnt += (uint32_t)~cr & MAX_LEAF;
+    }
+    hl = hl && !lf;
+    hr = hr && !rf;
+    return true;
+}
+
+// The xprim BVH (binary, `xnodes`, leaves of xprims) against [tmin, best_t]: updates best_t / best_item and
 // returns whether any hit is held.  Same node layout and walk as the binary traversal below.
 template <bool EXACT>
 __device__ __forceinline__ bool closest_hit_xprims(const DevScene& S, V3 o, V3 d, V3 inv, V3 oi, float tmin,
@@ -632,6 +647,7 @@ __device__ __forceinline__ bool closest_hit_xprims(const DevScene& S, V3 o, V3 d
     int32_t stack[TRAVERSAL_STACK];
     int sp = 0;
     int32_t node = 0;
+    XformRay xr{-1, o, d};
     for (;;) {
         const float4* np = S.xnodes + 4 * (size_t)node;
         float4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3);
@@ -640,8 +656,9 @@ __device__ __forceinline__ bool closest_hit_xprims(const DevScene& S, V3 o, V3 d
         float tl, tr;
         bool hr;
         bool hl = slab2(n0, n1, n2, inv, oi, tmin, best_t, tl, tr, hr);
-        if (hl && cl < 0) { test_leaf_xprims<EXACT>(S, cl, o, d, tmin, best_t, best_item, st, status); hl = false; }
-        if (hr && cr < 0) { test_leaf_xprims<EXACT>(S, cr, o, d, tmin, best_t, best_item, st, status); hr = false; }
+        uint32_t first, cnt, word;
+        if (hit_leaves(cl, cr, 0u, 0u, hl, hr, first, cnt, word))
+            test_xprims<EXACT>(S, first, cnt, o, d, xr, tmin, best_t, best_item, st, status);
         if (hl && hr) {
             int32_t nearc = tl <= tr ? cl : cr;
             int32_t farc = tl <= tr ? cr : cl;
@@ -661,10 +678,23 @@ __device__ __forceinline__ bool closest_hit_xprims(const DevScene& S, V3 o, V3 d
     return best_item != 0xffffffffu;
 }
 
+// Which node layouts a kernel's closest_hit walks.
+enum Walk { WALK_BINARY = 0, WALK_WIDE = 1, WALK_EITHER = 2 };   // EITHER: the 8-wide nodes of scenes that carry them
+
 // Closest hit in [tmin, tmax] over the whole scene (the reference's world.hit through the BVH).
-// EXACT: clean mode (double-precision sphere test).  WIDE: walk the 8-wide nodes when the scene
-// carries them (only the extend kernel is built with it, so the other kernels carry no code for it).
-template <bool EXACT = false, bool WIDE = false>
+// EXACT: clean mode (double-precision sphere test).  Only the extend kernel is built with the 8-wide walk
+// (the other kernels carry no code for it), and one image's without the binary one, whose registers it
+// would carry as well.
+//
+// The binary walk is bound by instruction issue and by the latency of dependent node fetches at a third of
+// the lanes.  Testing a visit's hit leaves as one range (hit_leaves) and finding their primitives without
+// the item list took the extend kernel from 30.2 to 27.1 ms on the spheres frame (489 primitives, 196 M
+// rays: 66.7 -> 59.5 M warp instructions in one launch) and from 57.7 to 48.9 ms on a 1.31 M triangle frame
+// (1920x1080, 16 spp), where the list was one more dependent miss per leaf.  Measured and left out: child
+// entry distances on the stack to skip popped nodes behind the best hit (3% fewer visits, 3% slower), leaves
+// deferred until half a warp holds one (spheres 35 ms), idle lanes refilled from a pool of rays with the
+// tree in shared memory (36-40 ms).
+template <bool EXACT = false, int WALK = WALK_BINARY>
 __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float tmin, float tmax,
                                             bool hide_invisible, float& t_out, uint32_t& item_out,
                                             TraceStats& st, uint32_t& status) {
@@ -677,8 +707,8 @@ __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float
         return false;
     }
     V3 inv = v3(1.0f / slab_dir(d.x), 1.0f / slab_dir(d.y), 1.0f / slab_dir(d.z));
-    if constexpr (WIDE) {
-        if (S.nodes8) {
+    if constexpr (WALK != WALK_BINARY) {
+        if (WALK == WALK_WIDE || S.nodes8) {
             V3 oi8 = v3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
             bool h = closest_hit8<EXACT>(S, o, d, inv, oi8, tmin, tmax, hide_invisible, t_out, item_out, st, status);
 #if RTC_XP
@@ -687,49 +717,53 @@ __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float
             return h;
         }
     }
-    V3 oi = v3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-    float best_t = tmax;
-    uint32_t best_item = 0xffffffffu;
-    int32_t stack[TRAVERSAL_STACK];
-    int sp = 0;
-    int32_t node = 0;
-    for (;;) {
+    if constexpr (WALK != WALK_WIDE) {
+        V3 oi = v3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
+        float best_t = tmax;
+        uint32_t best_item = 0xffffffffu;
+        int32_t stack[TRAVERSAL_STACK];
+        int sp = 0;
+        int32_t node = 0;
 #if RTC_XP
-        if (S.num_nodes == 0) break;   // every primitive is transformed (xprim BVH only)
+        if (S.num_nodes != 0)   // 0: every primitive is transformed (xprim BVH only)
 #endif
-        const float4* np = S.nodes + 4 * (size_t)node;
-        float4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3);
-        st.nodes++;
-        int32_t cl = __float_as_int(n3.x), cr = __float_as_int(n3.y);
-        float tl, tr;
-        bool hr;
-        bool hl = slab2(n0, n1, n2, inv, oi, tmin, best_t, tl, tr, hr);
-        if (hl && cl < 0) { test_leaf<EXACT>(S, cl, o, d, tmin, best_t, best_item, hide_invisible, st, status); hl = false; }
-        if (hr && cr < 0) { test_leaf<EXACT>(S, cr, o, d, tmin, best_t, best_item, hide_invisible, st, status); hr = false; }
-        if (hl && hr) {
-            int32_t nearc = tl <= tr ? cl : cr;
-            int32_t farc = tl <= tr ? cr : cl;
-            if (sp >= TRAVERSAL_STACK) { status |= STATUS_STACK_OVERFLOW; break; }
-            stack[sp++] = farc;
-            node = nearc;
-        } else if (hl) {
-            node = cl;
-        } else if (hr) {
-            node = cr;
-        } else {
-            if (sp == 0) break;
-            node = stack[--sp];
+        for (;;) {
+            const float4* np = S.nodes + 4 * (size_t)node;
+            float4 n0 = ld_scene(np), n1 = ld_scene(np + 1), n2 = ld_scene(np + 2), n3 = ld_scene(np + 3);
+            st.nodes++;
+            int32_t cl = __float_as_int(n3.x), cr = __float_as_int(n3.y);
+            float tl, tr;
+            bool hr;
+            bool hl = slab2(n0, n1, n2, inv, oi, tmin, best_t, tl, tr, hr);
+            uint32_t first, cnt, word;
+            if (hit_leaves(cl, cr, __float_as_uint(n3.z), __float_as_uint(n3.w), hl, hr, first, cnt, word))
+                test_items<EXACT>(S, S.items, first, cnt, word, o, d, tmin, best_t, best_item, hide_invisible, st, status);
+            if (hl && hr) {
+                int32_t nearc = tl <= tr ? cl : cr;
+                int32_t farc = tl <= tr ? cr : cl;
+                if (sp >= TRAVERSAL_STACK) { status |= STATUS_STACK_OVERFLOW; break; }
+                stack[sp++] = farc;
+                node = nearc;
+            } else if (hl) {
+                node = cl;
+            } else if (hr) {
+                node = cr;
+            } else {
+                if (sp == 0) break;
+                node = stack[--sp];
+            }
+            if ((uint32_t)node >= S.num_nodes) { status |= STATUS_BAD_ITEM; break; }
         }
-        if ((uint32_t)node >= S.num_nodes) { status |= STATUS_BAD_ITEM; break; }
-    }
-    t_out = best_t;
-    item_out = best_item;
-    // transformed primitives and box faces live in their own BVH, walked after the first one against the
-    // best hit so far; scenes without them skip it (and their traversal loop carries none of its registers)
+        t_out = best_t;
+        item_out = best_item;
+        // transformed primitives and box faces live in their own BVH, walked after the first one against the
+        // best hit so far; scenes without them skip it (and their traversal loop carries none of its registers)
 #if RTC_XP
-    if (S.num_xnodes) return closest_hit_xprims<EXACT>(S, o, d, inv, oi, tmin, t_out, item_out, st, status);
+        if (S.num_xnodes) return closest_hit_xprims<EXACT>(S, o, d, inv, oi, tmin, t_out, item_out, st, status);
 #endif
-    return best_item != 0xffffffffu;
+        return best_item != 0xffffffffu;
+    }
+    return false;
 }
 
 // Full hit record of the winning item: the part of each reference hit() that runs after the

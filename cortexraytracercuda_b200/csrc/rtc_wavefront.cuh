@@ -465,7 +465,8 @@ __global__ void __launch_bounds__(128) wf_admit(WfTable J, WfBuffers B, WfIter w
 }
 
 // FLAVOR: 0 nvcc flavour, 1 g++ flavour, 2 clean mode (double-precision sphere test).
-// WIDE: the 8-wide node layout (RTC_FLAG_WIDE_BVH; the other kernels always walk the binary nodes).
+// WIDE: the 8-wide node layout (RTC_FLAG_WIDE_BVH; the other kernels always walk the binary nodes).  One
+// image is rendered with it only when its scene carries it; a ring may mix scenes with and without.
 template <bool COUNT, int FLAVOR, class J, bool WIDE, bool DYN>
 __global__ void RTC_EXTEND_BOUNDS wf_extend(J jobs, WfBuffers B, WfIter w, unsigned long long* counters,
                                                  uint32_t* status_word) {
@@ -490,7 +491,8 @@ __global__ void RTC_EXTEND_BOUNDS wf_extend(J jobs, WfBuffers B, WfIter w, unsig
             const uint32_t job = wf_job(mw);
             float t;
             uint32_t item;
-            bool h = closest_hit<FLAVOR == 2, WIDE>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), wf_tmin(sec_f(R, 6)),
+            constexpr int WALK = !WIDE ? WALK_BINARY : std::is_same<J, WfOne>::value ? WALK_WIDE : WALK_EITHER;
+            bool h = closest_hit<FLAVOR == 2, WALK>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), wf_tmin(sec_f(R, 6)),
                                                     3.402823466e+38f,
                                                     wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t, item, st,
                                                     status);
