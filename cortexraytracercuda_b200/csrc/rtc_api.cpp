@@ -1141,14 +1141,11 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     // drain threshold: below this many queued slots the finish kernel takes over
     uint32_t drain = (uint32_t)num_sms * 512u;
     if (const char* ev = std::getenv("RTC_WF_DRAIN")) drain = (uint32_t)std::strtoul(ev, nullptr, 10);
-    // Drain kernel: one thread per slot for its whole chain, or the compacting drain, whose live slots
-    // are repacked into full warps every 2 bounce steps.  A frame with fewer work units than the drain
-    // threshold runs almost whole in the drain, where its short chains leave the lanes idle: there the
-    // compacting drain pays (Cornell 256x256, 16 spp: drain 1.91 -> 1.52 ms).  In a larger frame the
-    // drain is bound by its longest chains' bounce latency, which packing does not shorten (spheres
-    // frame: 19.0 against 18.6-19.4 ms), and its barriers cost a DRAM-bound walk (meshes frame: 67.7
-    // against 98.9 ms), so it keeps the plain drain.
-    L.drain_every = rtc_drain_every(P.num_pixels * (int64_t)P.groups <= (int64_t)drain ? 2 : 0);
+    // Drain kernel: one thread per slot, or the compacting drain, whose live slots are repacked into full
+    // warps every 2 bounce steps, for scenes with transformed primitives: their two walks and transforms
+    // make a bounce instruction-bound, where packing pays (5-15% of a frame at 16 or more spp); elsewhere
+    // the longest chains' latency bounds the drain and repacking costs 2-50% (wf_finish, wf_finish_packed).
+    L.drain_every = rtc_drain_every(S.num_xnodes ? 2 : 0);
     // Queue chunks handed out by a counter for scenes of 2^20 primitives or more, whose walks are long
     // and uneven (meshes frame, 1.31 M triangles: extend 450.7 -> 405.5 ms, 436 -> 460-467 Mpaths/s);
     // the fixed grid stride for smaller ones (spheres frame, 489 primitives: 945 against 840 Mpaths/s;
@@ -1161,7 +1158,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     float split_thr = 1024.0f;
     if (const char* ev = std::getenv("RTC_WF_SPLIT")) split_at = std::strtoull(ev, nullptr, 10);
     if (const char* ev = std::getenv("RTC_WF_SPLIT_THRESH")) split_thr = std::strtof(ev, nullptr);
-    int split_blocks = 1;   // blocks per SM of the long-chain kernel (its registers stay taken while it runs)
+    int split_blocks = 1;   // 128 threads per SM each of the long-chain kernel (its registers stay taken while it runs)
     if (const char* ev = std::getenv("RTC_WF_SPLIT_BLOCKS")) split_blocks = std::max(1, std::atoi(ev));
     int64_t last_left = -1;   // queue size last observed (one batch late in both polling modes)
     // split extend / shade kernels (default) or one fused launch per iteration
@@ -1208,7 +1205,8 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
             run.split = true;
             WfLaunch LL = L;
             LL.w = WfIter{2, WF_LONG, 0, 0};
-            LL.grid = num_sms * split_blocks;
+            LL.grid = num_sms * split_blocks * (128 / rtc::WF_FINISH_BLOCK);
+            LL.drain_every = 0;
             LL.st = poll.st_long ? poll.st_long : st;
             if (poll.st_long) {
                 RTC_CUDA(cudaEventRecord(poll.split_ev[0], st));
@@ -1262,7 +1260,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     if (phase) RTC_CUDA(cudaEventRecord(phase[1], st));
     if (run.drained) {
         L.w = wf_iter(it);
-        const uint32_t per_block = L.drain_every > 0 ? (uint32_t)rtc::WF_DRAIN_BLOCK : 128u;
+        const uint32_t per_block = L.drain_every > 0 ? (uint32_t)rtc::WF_DRAIN_BLOCK : (uint32_t)rtc::WF_FINISH_BLOCK;
         L.grid = (int)std::max<uint32_t>(1u, (drain + per_block - 1u) / per_block);
         e = fn(WF_OP_FINISH, J, B, L);
         if (e != cudaSuccess) return cuda_fail(e, "wavefront finish");

@@ -24,6 +24,7 @@
 #endif
 
 namespace rtc {
+constexpr int WF_FINISH_BLOCK = 32;   // threads per block of the drain (wf_finish)
 constexpr int WF_DRAIN_BLOCK = 256;   // threads per block of the compacting drain (wf_finish_packed)
 
 // Wavefront kernel launches.  One dispatcher per (mode, flavour) and job source; `op` picks the kernel.
@@ -42,9 +43,8 @@ struct WfLaunch {
     int block;                       // EXTEND / SHADE / BOUNCE: threads per block (0: 128; at most 512)
     bool dynamic;                    // EXTEND / SHADE: warps take chunks of the queue from a counter (WfChunks)
                                      // instead of a fixed grid stride
-    int drain_every;                 // FINISH: 0 the plain drain (128-thread blocks, one thread per slot);
-                                     // k > 0 the compacting drain (256-thread blocks, live slots repacked
-                                     // every k bounce steps)
+    int drain_every;                 // FINISH: 0 the drain (one thread per slot); k > 0 the compacting drain
+                                     // (256-thread blocks, live slots repacked every k bounce steps)
     cudaStream_t st;
 };
 using WfOneFn = cudaError_t (*)(WfOp, const WfOneArgs&, const WfBuffers&, const WfLaunch&);

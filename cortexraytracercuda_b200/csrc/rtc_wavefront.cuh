@@ -45,11 +45,6 @@
 #endif
 #define RTC_SHADE_BOUNDS __maxnreg__(RTC_SHADE_MAXNREG)
 #endif
-#ifdef RTC_FINISH_MINB
-#define RTC_FINISH_BOUNDS __launch_bounds__(128, RTC_FINISH_MINB)
-#else
-#define RTC_FINISH_BOUNDS __launch_bounds__(128)
-#endif
 
 #include "rtc_kernels.h"
 #include "rtc_path.cuh"
@@ -745,90 +740,8 @@ __global__ void __launch_bounds__(128) wf_split(J jobs, WfBuffers B, WfIter w, f
 // Drain phase: once the queue is small, each remaining slot is finished in place by one thread
 // instead of paying two kernel launches per bounce for a nearly empty queue.  Pixels whose samples
 // have long paths (glass) make this tail thousands of bounces long in compat mode, where a pixel's
-// samples cannot run in parallel, so the loop keeps the whole path state in registers (the
-// megakernel's loop, resumed from the slot) and touches memory only to write the finished pixel.
-template <bool CLEAN, int ORDER, bool COUNT, class J>
-__global__ void RTC_FINISH_BOUNDS wf_finish(J jobs, WfBuffers B, WfIter w, unsigned long long* counters,
-                                                 uint32_t* status_word) {
-    const uint32_t n = B.ctr[w.cin];
-    const WfWindow win = jobs.window();
-    const uint32_t* q = B.queue[w.qin];
-    uint32_t status = 0, paths = 0;
-    PathCounters pc{0, 0, 0};
-    TraceStats st{0, 0};
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
-        const uint32_t slot = ld_state(q + k);
-        const Sec R = ld_sec(wf_sec(B, slot, SEC_RAY)), SH = ld_sec(wf_sec(B, slot, SEC_SHADE)),
-                  PX = ld_sec(wf_sec(B, slot, SEC_PIXEL));
-        Ray r;
-        r.o = sec_v3(R, 0);
-        r.d = sec_v3(R, 3);
-        r.time = 0.0f;
-        RGB att = rgb(sec_f(SH, 0), sec_f(SH, 1), sec_f(SH, 2)), acc = rgb(sec_f(SH, 3), sec_f(SH, 4), sec_f(SH, 5));
-        const float4 p4 = sec_psum(PX);
-        float pr = p4.x, pg = p4.y, pb = p4.z;
-        WfRng<CLEAN> rng;
-        rng_load<CLEAN>(PX, rng);
-        uint32_t pixel = PX.w[0], sample = PX.w[1], job = wf_job(R.w[7]), grp = CLEAN ? PX.w[2] : 0u;
-        int depth = (int)wf_depth(R.w[7]);
-        float tmin = wf_tmin(sec_f(R, 6));   // the slot may wait for its re-hit from behind a one-sided light
-        // one pass of the loop finishes the current sample of the current pixel
-        for (;;) {
-            const DevScene& S = jobs.scene(job);
-            const DevParams& P = jobs.params(job);
-            // the rest of the current sample: camera::ray_color's loop from `depth` down
-            trace_bounces<CLEAN, ORDER>(S, r, depth, P.max_depth, tmin, acc, att, rng, pc, st, status);
-            ++paths;
-            if (!CLEAN || (isfinite(acc.r) && isfinite(acc.g) && isfinite(acc.b))) {
-                pr += acc.r;
-                pg += acc.g;
-                pb += acc.b;
-            }
-            if (++sample < (P.groups > 1 ? wf_group_end(P, grp, CLEAN) : wf_samples(P, CLEAN))) {
-                wf_start_sample<CLEAN, ORDER>(S, P, rng, pixel, sample, r);
-                att = rgb(1.f, 1.f, 1.f);
-                acc = rgb(0.f, 0.f, 0.f);
-                depth = P.max_depth;
-                tmin = 0.00001f;
-                continue;
-            }
-            wf_group_done(jobs, job, pixel, grp, make_float4(pr, pg, pb, 0.0f));
-            // a slot that still has pixels to take (fewer slots than pixels) continues through memory
-            if (!wf_fetch_pixel<CLEAN, ORDER>(jobs, win, B, slot, status)) break;
-            const Sec R2 = ld_sec(wf_sec(B, slot, SEC_RAY)), PX2 = ld_sec(wf_sec(B, slot, SEC_PIXEL));
-            r.o = sec_v3(R2, 0);
-            r.d = sec_v3(R2, 3);
-            att = rgb(1.f, 1.f, 1.f);
-            acc = rgb(0.f, 0.f, 0.f);
-            pr = pg = pb = 0.f;
-            rng_load<CLEAN>(PX2, rng);
-            pixel = PX2.w[0];
-            sample = PX2.w[1];
-            grp = CLEAN ? PX2.w[2] : 0u;
-            job = wf_job(R2.w[7]);
-            depth = (int)wf_depth(R2.w[7]);
-            tmin = wf_tmin(sec_f(R2, 6));
-            if (status) break;
-        }
-    }
-    wf_flush<COUNT>(counters, pc.rays, paths, st);
-    if (status) atomicOr(status_word, status);
-}
-
-// Compacting drain.  The plain drain above gives each remaining slot one thread for its whole chain,
-// so a warp runs as long as its longest chain while its other lanes idle (3.8 of 32 lanes active on
-// the spheres frame).  Here the chains advance one bounce per step, and every `every` steps the live
-// slots of a block move, through shared memory, to the block's lowest threads: the live chains stay
-// packed into full warps, and the warps left without a slot wait at the block barrier without
-// issuing.  Each slot computes exactly what the plain drain computes for it (the same bounce, sample
-// and pixel code in the same order); only which thread runs it changes.
-//
-// A block takes the queue entries b, b + G, b + 2G, ... (G blocks), so pixels that sit together in the
-// queue - neighbours, with similar chains - spread over all SMs; entries past G x WF_DRAIN_BLOCK are
-// taken in further rounds.
-constexpr int WF_DRAIN_WORDS = 23;   // a slot's state in the pool (WF_DRAIN_BLOCK: rtc_kernels.h)
-
+// samples cannot run in parallel, so the path state stays in registers and memory is touched only to
+// write the finished pixel.
 template <bool CLEAN>
 struct DrainSlot {
     V3 o, d;
@@ -859,54 +772,9 @@ __device__ __forceinline__ void drain_load(const WfBuffers& B, uint32_t slot, Dr
     x.slot = slot;
 }
 
-// the slot's words in (or out of) the block's shared pool, column `i`
-template <bool CLEAN>
-__device__ __forceinline__ void drain_put(uint32_t (*pool)[WF_DRAIN_BLOCK], int i, const DrainSlot<CLEAN>& x) {
-    const float f[16] = {x.o.x, x.o.y, x.o.z, x.d.x, x.d.y, x.d.z, x.tmin, x.att.r, x.att.g, x.att.b,
-                         x.acc.r, x.acc.g, x.acc.b, x.pr, x.pg, x.pb};
-#pragma unroll
-    for (int k = 0; k < 16; ++k) pool[k][i] = __float_as_uint(f[k]);
-    pool[16][i] = x.pixel;
-    pool[17][i] = x.sample;
-    pool[18][i] = x.mw;
-    pool[19][i] = x.grp;
-    pool[20][i] = x.slot;
-    if constexpr (CLEAN) {
-        pool[21][i] = (uint32_t)x.rng.state;
-        pool[22][i] = (uint32_t)(x.rng.state >> 32);
-    } else {
-        pool[21][i] = x.rng.x;
-    }
-}
-template <bool CLEAN>
-__device__ __forceinline__ void drain_get(uint32_t (*pool)[WF_DRAIN_BLOCK], int i, DrainSlot<CLEAN>& x) {
-    float f[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(pool[k][i]);
-    x.o = v3(f[0], f[1], f[2]);
-    x.d = v3(f[3], f[4], f[5]);
-    x.tmin = f[6];
-    x.att = rgb(f[7], f[8], f[9]);
-    x.acc = rgb(f[10], f[11], f[12]);
-    x.pr = f[13];
-    x.pg = f[14];
-    x.pb = f[15];
-    x.pixel = pool[16][i];
-    x.sample = pool[17][i];
-    x.mw = pool[18][i];
-    x.grp = pool[19][i];
-    x.slot = pool[20][i];
-    if constexpr (CLEAN) {
-        x.rng.state = ((uint64_t)pool[22][i] << 32) | pool[21][i];
-        x.rng.inc = ((uint64_t)x.sample << 1) | 1u;
-    } else {
-        x.rng.x = pool[21][i];
-    }
-}
-
 // One step of a slot: one pass of camera::ray_color's loop body (trace, then shade_bounce_deferred),
-// then the sample's and the pixel's bookkeeping when the sample ends - trace_bounces and the plain
-// drain's loop, one bounce at a time.  Returns false when the slot has no pixel left.
+// then the sample's and the pixel's bookkeeping when the sample ends - trace_bounces, one bounce at a
+// time.  Returns false when the slot has no pixel left.
 template <bool CLEAN, int ORDER, class J>
 __device__ __forceinline__ bool drain_step(const J& jobs, const WfWindow& win, const WfBuffers& B, DrainSlot<CLEAN>& x,
                                            PathCounters& pc, TraceStats& st, uint32_t& paths, uint32_t& status) {
@@ -960,6 +828,97 @@ __device__ __forceinline__ bool drain_step(const J& jobs, const WfWindow& win, c
     return status == 0u;
 }
 
+// The drain: one slot per thread, one bounce per trip of the loop, whatever sample each lane is in.  (A loop
+// over whole samples made every lane wait, sample by sample, for the warp's longest path: 3.8 of 32 lanes
+// active.)  Blocks are single warps and thread t of block b takes queue entry b + t x G (G blocks), so
+// neighbouring pixels, whose chains are alike, sit in different warps: every warp gets its share of long
+// chains, and a warp's registers are free as soon as its own chains end.  What bounds it is the latency of
+// a warp's dependent bounces, about 6 us each, over the longest chain (1,952 bounces after the start of the
+// drain on the spheres frame).  Drain time against the loop over samples in 128-thread blocks of
+// neighbours: spheres 1280x720 18.5 -> 13.0 ms, meshes (1.31 M triangles) 8.6 -> 6.4, Cornell 256x256
+// 1.34 -> 1.21 (with the compacting drain before), 16-image batch 26.4 -> 25.1 ms in all; blocks of 64 and
+// 128 neighbours: spheres 13.3 and 13.6, meshes 7.1 and 7.6 ms.  More resident warps do not pay: 20 per SM
+// (96 registers) 14.1 ms.
+template <bool CLEAN, int ORDER, bool COUNT, class J>
+__global__ void __launch_bounds__(WF_FINISH_BLOCK, 16) wf_finish(J jobs, WfBuffers B, WfIter w,
+                                                                 unsigned long long* counters, uint32_t* status_word) {
+    const uint32_t n = B.ctr[w.cin];
+    const WfWindow win = jobs.window();
+    const uint32_t* q = B.queue[w.qin];
+    uint32_t status = 0, paths = 0;
+    PathCounters pc{0, 0, 0};
+    TraceStats st{0, 0};
+    for (uint32_t round = 0; round < n; round += gridDim.x * WF_FINISH_BLOCK) {
+        DrainSlot<CLEAN> x;
+        const uint32_t k = round + blockIdx.x + gridDim.x * threadIdx.x;
+        bool live = k < n;
+        if (live) drain_load<CLEAN>(B, ld_state(q + k), x);
+        while (__any_sync(0xffffffffu, live))   // the lanes meet after every bounce
+            if (live) live = drain_step<CLEAN, ORDER>(jobs, win, B, x, pc, st, paths, status);
+    }
+    wf_flush<COUNT>(counters, pc.rays, paths, st);
+    if (status) atomicOr(status_word, status);
+}
+
+// Compacting drain.  Every `every` steps the live slots of a 256-thread block move, through shared memory,
+// to the block's lowest threads: the live chains stay packed into full warps, and the warps left without a
+// slot wait at the block barrier without issuing.  Each slot computes exactly what the drain above computes
+// for it (the same step in the same order); only which thread runs it changes.  It pays where a bounce is
+// bound by instructions rather than by the latency of the longest chain: scenes with transformed primitives
+// (the second walk and the transforms; 333x251, 32 spp, clean: drain 5.5 -> 4.7 ms; 5-15% of the frame at
+// 30-235 K pixels and 16 or more spp).  Elsewhere the barriers and the dense tail cost: 2-8% of the frame on
+// small scenes, 25-50% on triangle meshes.
+//
+// A block takes the queue entries b, b + G, b + 2G, ... (G blocks), so pixels that sit together in the
+// queue - neighbours, with similar chains - spread over all SMs; entries past G x WF_DRAIN_BLOCK are
+// taken in further rounds.
+constexpr int WF_DRAIN_WORDS = 23;   // a slot's state in the pool (WF_DRAIN_BLOCK: rtc_kernels.h)
+
+// the slot's words in (or out of) the block's shared pool, column `i`
+template <bool CLEAN>
+__device__ __forceinline__ void drain_put(uint32_t (*pool)[WF_DRAIN_BLOCK], int i, const DrainSlot<CLEAN>& x) {
+    const float f[16] = {x.o.x, x.o.y, x.o.z, x.d.x, x.d.y, x.d.z, x.tmin, x.att.r, x.att.g, x.att.b,
+                         x.acc.r, x.acc.g, x.acc.b, x.pr, x.pg, x.pb};
+#pragma unroll
+    for (int k = 0; k < 16; ++k) pool[k][i] = __float_as_uint(f[k]);
+    pool[16][i] = x.pixel;
+    pool[17][i] = x.sample;
+    pool[18][i] = x.mw;
+    pool[19][i] = x.grp;
+    pool[20][i] = x.slot;
+    if constexpr (CLEAN) {
+        pool[21][i] = (uint32_t)x.rng.state;
+        pool[22][i] = (uint32_t)(x.rng.state >> 32);
+    } else {
+        pool[21][i] = x.rng.x;
+    }
+}
+template <bool CLEAN>
+__device__ __forceinline__ void drain_get(uint32_t (*pool)[WF_DRAIN_BLOCK], int i, DrainSlot<CLEAN>& x) {
+    float f[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) f[k] = __uint_as_float(pool[k][i]);
+    x.o = v3(f[0], f[1], f[2]);
+    x.d = v3(f[3], f[4], f[5]);
+    x.tmin = f[6];
+    x.att = rgb(f[7], f[8], f[9]);
+    x.acc = rgb(f[10], f[11], f[12]);
+    x.pr = f[13];
+    x.pg = f[14];
+    x.pb = f[15];
+    x.pixel = pool[16][i];
+    x.sample = pool[17][i];
+    x.mw = pool[18][i];
+    x.grp = pool[19][i];
+    x.slot = pool[20][i];
+    if constexpr (CLEAN) {
+        x.rng.state = ((uint64_t)pool[22][i] << 32) | pool[21][i];
+        x.rng.inc = ((uint64_t)x.sample << 1) | 1u;
+    } else {
+        x.rng.x = pool[21][i];
+    }
+}
+
 template <bool CLEAN, int ORDER, bool COUNT, class J>
 __global__ void __launch_bounds__(WF_DRAIN_BLOCK, 2) wf_finish_packed(J jobs, WfBuffers B, WfIter w, int every,
                                                                   unsigned long long* counters, uint32_t* status_word) {
@@ -980,7 +939,7 @@ __global__ void __launch_bounds__(WF_DRAIN_BLOCK, 2) wf_finish_packed(J jobs, Wf
         bool live = k < n;
         if (live) drain_load<CLEAN>(B, ld_state(q + k), x);
         for (;;) {
-            for (int s = 0; s < steps; ++s)
+            for (int s = 0; s < steps && __any_sync(0xffffffffu, live); ++s)
                 if (live) live = drain_step<CLEAN, ORDER>(jobs, win, B, x, pc, st, paths, status);
             // compaction: the live slots move to threads 0 .. total-1, in thread order
             const unsigned m = __ballot_sync(0xffffffffu, live);
@@ -1063,8 +1022,8 @@ cudaError_t wf_dispatch(WfOp op, const A& args, const WfBuffers& B, const WfLaun
             else wf_finish_packed<CLEAN, ORDER, false><<<L.grid, WF_DRAIN_BLOCK, 0, L.st>>>(jobs, B, L.w, L.drain_every,
                                                                                             nullptr, L.status);
         } else {
-            if (c) wf_finish<CLEAN, ORDER, true><<<L.grid, 128, 0, L.st>>>(jobs, B, L.w, L.counters, L.status);
-            else wf_finish<CLEAN, ORDER, false><<<L.grid, 128, 0, L.st>>>(jobs, B, L.w, nullptr, L.status);
+            if (c) wf_finish<CLEAN, ORDER, true><<<L.grid, WF_FINISH_BLOCK, 0, L.st>>>(jobs, B, L.w, L.counters, L.status);
+            else wf_finish<CLEAN, ORDER, false><<<L.grid, WF_FINISH_BLOCK, 0, L.st>>>(jobs, B, L.w, nullptr, L.status);
         }
         break;
     case WF_OP_SPLIT:

@@ -1,0 +1,36 @@
+"""The drain kernels finish exactly the slots they are given, whatever their number: the wavefront engine
+against the megakernel, g++ flavour (no FMA contraction: the sums are identical), at sizes around a warp, a
+block of the compacting drain and the number of drain threads (75,776), with chains of one bounce to many.
+Scenes without transforms run the drain of one-warp blocks, scenes with them the compacting drain."""
+import numpy as np
+import pytest
+
+from cortexraytracercuda_b200 import configs
+from cortexraytracercuda_b200.renderer import DeviceScene
+from cortexraytracercuda_b200.scene import (DRAW_ORDER_HOST, ENGINE_MEGAKERNEL, ENGINE_WAVEFRONT, MODE_CLEAN,
+                                            FLAG_SAMPLE_GROUPS, RenderParams)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("name", ["textured", "xforms"])
+@pytest.mark.parametrize("w,h,spp,depth", [(1, 1, 9, 50), (31, 1, 4, 20), (33, 1, 4, 20), (257, 1, 9, 12), (64, 37, 16, 1),
+                                           (275, 276, 9, 10)])
+def test_drain_equals_megakernel(ctx, name, w, h, spp, depth):
+    ds = DeviceScene(ctx, configs.SCENES[name][0]())
+    p = RenderParams(width=w, height=h, spp=spp, max_depth=depth, draw_order=DRAW_ORDER_HOST, engine=ENGINE_MEGAKERNEL)
+    a, rgb_a = ds.render(p, want_rgb8=True)
+    p.engine = ENGINE_WAVEFRONT
+    b, rgb_b = ds.render(p, want_rgb8=True)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    assert np.array_equal(rgb_a, rgb_b)
+
+
+@pytest.mark.parametrize("name", ["textured", "xforms"])
+def test_drain_sample_groups_repeatable(ctx, name):
+    """Sample groups through the drains: every group finishes once and is added in group order."""
+    ds = DeviceScene(ctx, configs.SCENES[name][0]())
+    p = RenderParams(width=97, height=41, spp=13, max_depth=9, mode=MODE_CLEAN, flags=FLAG_SAMPLE_GROUPS)
+    a, _ = ds.render(p)
+    b, _ = ds.render(p)
+    assert np.array_equal(a.view(np.uint32), b.view(np.uint32)) and np.isfinite(a).all()
