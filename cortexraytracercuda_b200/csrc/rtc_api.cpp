@@ -1068,7 +1068,7 @@ struct WfPoller {
 };
 
 struct WfRun {
-    uint64_t iterations = 0;
+    uint64_t iterations = 0, launches = 0;
     bool drained = false;
     uint32_t drained_slots = 0;
     bool split = false;
@@ -1107,6 +1107,11 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
                          float4* d_out, unsigned long long* d_counters, cudaStream_t st, int num_sms,
                          const WfPoller& poll, cudaEvent_t* phase, WfRun& run, WfTimer* timer = nullptr,
                          void* groups = nullptr, uint8_t* d_rgb8 = nullptr) {
+    // A render shares its context's scratch (or the static array) with the renders after it and polls its
+    // queue, so it cannot be captured; a frame short enough to need no poll is refused like any other.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    RTC_CUDA(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return fail(RTC_ERR_CUDA, "a render cannot be captured into a graph");
     DevParams P = dev_params(p);
     P.rgb8 = d_rgb8;   // quantised output written as each pixel finishes
     const bool clean = p->mode == RTC_MODE_CLEAN;
@@ -1133,6 +1138,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     L.grid = (int)std::min<int64_t>((B.slots + 127) / 128, (int64_t)num_sms * 16);
     cudaError_t e = fn(WF_OP_INIT, J, B, L);
     if (e != cudaSuccess) return cuda_fail(e, "wavefront init");
+    run.launches = 1;
     L.grid = grid;
     const uint64_t nsamp = clean ? (uint64_t)P.spp : (uint64_t)P.sqrt_spp * P.sqrt_spp;
     const uint64_t rounds = (uint64_t)((P.num_pixels * P.groups + B.slots - 1) / B.slots);
@@ -1161,9 +1167,12 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     int split_blocks = 1;   // 128 threads per SM each of the long-chain kernel (its registers stay taken while it runs)
     if (const char* ev = std::getenv("RTC_WF_SPLIT_BLOCKS")) split_blocks = std::max(1, std::atoi(ev));
     int64_t last_left = -1;   // queue size last observed (one batch late in both polling modes)
-    // split extend / shade kernels (default) or one fused launch per iteration
-    bool fused = false;
-    if (const char* ev = std::getenv("RTC_WF_FUSED")) fused = std::atoi(ev) != 0;
+    // A batch of iterations over at most this many queued slots is one wf_bounces launch (see there); the
+    // instrumented and the timed forms and the 8-wide walk keep the split kernels.
+    uint32_t bounces_max = timer || d_counters || L.wide ? 0u : (uint32_t)num_sms * 2048u;
+    if (const char* ev = std::getenv("RTC_WF_BOUNCES")) bounces_max = std::min(bounces_max, (uint32_t)std::strtoul(ev, nullptr, 10));
+    const int64_t units = P.num_pixels * P.groups;
+    uint64_t rot = 0;   // queue rotations: one per launch that reads one queue and fills the other
     uint64_t it = 0;
     int pending = -1;   // poll slot of the previous batch
     uint32_t left = 0;
@@ -1173,7 +1182,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
         const int slot = b & 1;
         if (poll.sync) {
             uint32_t h = 0;
-            RTC_CUDA(cudaMemcpyAsync(&h, B.ctr + wf_iter(it).cin, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+            RTC_CUDA(cudaMemcpyAsync(&h, B.ctr + wf_iter(rot).cin, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
             RTC_CUDA(cudaStreamSynchronize(st));
             sync_counts[slot] = h;
             if (pending >= 0) {
@@ -1181,7 +1190,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
                 have = true;
             }
         } else {
-            RTC_CUDA(cudaMemcpyAsync(poll.h + slot, B.ctr + wf_iter(it).cin, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+            RTC_CUDA(cudaMemcpyAsync(poll.h + slot, B.ctr + wf_iter(rot).cin, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                      st));
             RTC_CUDA(cudaEventRecord(poll.ev[slot], st));
             if (pending >= 0) {
@@ -1196,12 +1205,13 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     for (int b = 0;; ++b) {
         if (!run.split && split_at > 0 && it >= split_at && last_left >= (int64_t)drain) {
             // the split takes the place of one iteration (same queue rotation)
-            L.w = wf_iter(it);
+            L.w = wf_iter(rot++);
             L.k0 = (float)it;
             L.threshold = split_thr;
             e = fn(WF_OP_SPLIT, J, B, L);
             if (e != cudaSuccess) return cuda_fail(e, "wavefront split");
             ++it;
+            run.launches += 2;   // the split and the long chains' drain
             run.split = true;
             WfLaunch LL = L;
             LL.w = WfIter{2, WF_LONG, 0, 0};
@@ -1216,11 +1226,20 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
             if (e != cudaSuccess) return cuda_fail(e, "wavefront long chains");
             if (poll.st_long) RTC_CUDA(cudaEventRecord(poll.split_ev[1], poll.st_long));
         }
-        for (int k = 0; k < BATCH; ++k, ++it) {
-            L.w = wf_iter(it);
-            if (fused) {
-                e = fn(WF_OP_BOUNCE, J, B, L);
-            } else {
+        // the queue only shrinks while the units fit the slots (a finished unit's slot has none to take)
+        const int64_t bound = last_left >= 0 ? last_left : units;
+        if (units <= (int64_t)B.slots && bound <= (int64_t)bounces_max) {
+            L.w = wf_iter(rot++);
+            L.steps = BATCH;
+            L.grid = (int)std::max<int64_t>(1, (bound + rtc::WF_BOUNCES_BLOCK - 1) / rtc::WF_BOUNCES_BLOCK);
+            e = fn(WF_OP_BOUNCES, J, B, L);
+            L.grid = grid;
+            if (e != cudaSuccess) return cuda_fail(e, "wavefront iterations");
+            it += BATCH;
+            ++run.launches;
+        } else {
+            for (int k = 0; k < BATCH; ++k, ++it) {
+                L.w = wf_iter(rot++);
                 cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
                 if (timer) {
                     RTC_CUDA(timer->pair(e0, e1));
@@ -1238,8 +1257,17 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
                     RTC_CUDA(cudaEventRecord(e3, st));
                     timer->shade.push_back({e2, e3});
                 }
+                if (e != cudaSuccess) return cuda_fail(e, "wavefront iteration");
+                run.launches += 2;
             }
-            if (e != cudaSuccess) return cuda_fail(e, "wavefront iteration");
+        }
+        // A frame of fewer units than the drain threshold always drains after its second batch (the count of
+        // the first is at most the units): nothing to wait for.
+        if (bound <= (int64_t)bounces_max && units <= (int64_t)B.slots && units < (int64_t)drain && split_at == 0) {
+            if (b == 0) continue;
+            left = (uint32_t)units;
+            run.drained = true;
+            break;
         }
         // Both polling modes act on the count of the PREVIOUS batch (the next batch is already
         // queued when the host looks), so the drain point - and with it the result - does not depend
@@ -1259,11 +1287,12 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     run.drained_slots = run.drained ? left : 0u;
     if (phase) RTC_CUDA(cudaEventRecord(phase[1], st));
     if (run.drained) {
-        L.w = wf_iter(it);
+        L.w = wf_iter(rot);
         const uint32_t per_block = L.drain_every > 0 ? (uint32_t)rtc::WF_DRAIN_BLOCK : (uint32_t)rtc::WF_FINISH_BLOCK;
         L.grid = (int)std::max<uint32_t>(1u, (drain + per_block - 1u) / per_block);
         e = fn(WF_OP_FINISH, J, B, L);
         if (e != cudaSuccess) return cuda_fail(e, "wavefront finish");
+        ++run.launches;
     }
     if (run.split && poll.st_long) RTC_CUDA(cudaStreamWaitEvent(st, poll.split_ev[1], 0));   // long chains done
     if (phase) RTC_CUDA(cudaEventRecord(phase[2], st));
@@ -1307,12 +1336,10 @@ rtc_status launch_wavefront(rtc_context* c, const rtc_scene* s, const rtc_render
         for (auto& pr : timer.ext) c->kev_pairs.push_back(pr);
         for (auto& pr : timer.shade) c->kev_pairs.push_back(pr);
     }
-    const bool fused = std::getenv("RTC_WF_FUSED") && std::atoi(std::getenv("RTC_WF_FUSED")) != 0;
     c->last = rtc_render_stats{};
     c->last.engine = RTC_ENGINE_WAVEFRONT;
     c->last.iterations = (uint32_t)run.iterations;
-    // (the split pass counts as one iteration: the split launch and the long-chain drain launch)
-    c->last.launches = (uint32_t)(1 + (fused ? 1 : 2) * run.iterations + (run.drained ? 1 : 0));
+    c->last.launches = (uint32_t)run.launches;
     c->last.drained_slots = run.drained_slots;
     c->last_timed = true;
     return RTC_OK;

@@ -24,23 +24,25 @@
 #endif
 
 namespace rtc {
+constexpr int WF_BOUNCES_BLOCK = 32;  // threads per block of the several-iterations kernel (wf_bounces)
 constexpr int WF_FINISH_BLOCK = 32;   // threads per block of the drain (wf_finish)
 constexpr int WF_DRAIN_BLOCK = 256;   // threads per block of the compacting drain (wf_finish_packed)
 
 // Wavefront kernel launches.  One dispatcher per (mode, flavour) and job source; `op` picks the kernel.
 enum WfOp {
-    WF_OP_INIT = 0, WF_OP_ADMIT = 1, WF_OP_EXTEND = 2, WF_OP_SHADE = 3, WF_OP_FINISH = 4, WF_OP_BOUNCE = 5,
+    WF_OP_INIT = 0, WF_OP_ADMIT = 1, WF_OP_EXTEND = 2, WF_OP_SHADE = 3, WF_OP_FINISH = 4, WF_OP_BOUNCES = 5,
     WF_OP_SPLIT = 6
 };
 struct WfLaunch {
     WfIter w;
     WfWindow win;                    // ADMIT: the window to publish
+    int steps;                       // BOUNCES: bounces per slot
     float k0, threshold;             // SPLIT: iterations so far, long-chain threshold (iterations)
     bool wide;                       // EXTEND: walk the 8-wide nodes (where the scene carries them)
     unsigned long long* counters;    // NULL: no instrumentation
     uint32_t* status;
     int grid;
-    int block;                       // EXTEND / SHADE / BOUNCE: threads per block (0: 128; at most 512)
+    int block;                       // EXTEND / SHADE: threads per block (0: 128; at most 512)
     bool dynamic;                    // EXTEND / SHADE: warps take chunks of the queue from a counter (WfChunks)
                                      // instead of a fixed grid stride
     int drain_every;                 // FINISH: 0 the drain (one thread per slot); k > 0 the compacting drain

@@ -21,7 +21,7 @@
 
 #include <type_traits>
 
-// Launch bounds of the iteration kernels (extend, shade, fused bounce), which run with 128, 256 or 512
+// Launch bounds of the iteration kernels (extend, shade), which run with 128, 256 or 512
 // threads per block (WfLaunch::block, a batch autotuner knob).  Build-time knobs for occupancy sweeps:
 // RTC_EXTEND_MINB / RTC_SHADE_MINB ask for that many resident 512-thread blocks per SM (a register cap of
 // 65536 / (512 x blocks)), RTC_EXTEND_MAXNREG caps the extend kernel at any count.  Without them the
@@ -82,8 +82,17 @@ __device__ __forceinline__ uint32_t* wf_sec(const WfBuffers& B, uint32_t slot, i
     return B.rec + (size_t)slot * WF_REC_WORDS + 8 * sec;
 }
 
+// OWN: through L1, for a sector that this thread itself wrote in this kernel (wf_bounces).
+template <bool OWN = false>
 __device__ __forceinline__ Sec ld_sec(const uint32_t* p) {
     Sec s;
+    if constexpr (OWN) {
+        asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(s.w[0]), "=r"(s.w[1]), "=r"(s.w[2]), "=r"(s.w[3]), "=r"(s.w[4]), "=r"(s.w[5]), "=r"(s.w[6]),
+                       "=r"(s.w[7])
+                     : "l"(p));
+        return s;
+    }
 #if RTC_STATE_LOAD == 1
     asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
 #elif RTC_STATE_LOAD == 2
@@ -517,7 +526,7 @@ __global__ void RTC_EXTEND_BOUNDS wf_extend(J jobs, WfBuffers B, WfIter w, unsig
 
 // One shade step of a slot whose current ray has been traced: shade_bounce_deferred, then the slot's
 // bookkeeping (next bounce / next sample / next pixel).  Returns true while the slot has a ray to trace.
-template <bool CLEAN, int ORDER, class J>
+template <bool CLEAN, int ORDER, bool OWN = false, class J>
 __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, const WfBuffers& B, uint32_t slot,
                                         const Sec& R, const Sec& SH, const Sec& PX, float t, uint32_t item,
                                         PathCounters& pc, TraceStats& st, uint32_t& paths, uint32_t& status) {
@@ -565,7 +574,7 @@ __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, cons
     // the sample is done: pixel_color += ray_color(...) (gpu.cu:787).  The pixel sector is read again
     // here (a quarter of the bounces end a sample) rather than held in registers through the bounce.
     ++paths;
-    const Sec px = ld_sec(rec_px);
+    const Sec px = ld_sec<OWN>(rec_px);
     float4 ps = sec_psum(px);
     if (!CLEAN || (isfinite(acc.r) && isfinite(acc.g) && isfinite(acc.b))) {
         ps.x += acc.r;
@@ -666,42 +675,51 @@ __global__ void RTC_SHADE_BOUNDS wf_shade_ring(WfTable jobs, WfBuffers B, WfIter
     wf_shade_pass<CLEAN, ORDER, COUNT, DYN>(jobs, B, w, counters, status_word);
 }
 
-// Fused form of one iteration: trace + shade of every queued slot in one launch (each lane still does
-// exactly one bounce, so the warp stays in the same phase), then compaction into the next queue.
-template <bool CLEAN, int ORDER, bool COUNT, class J>
-__global__ void __launch_bounds__(RTC_ITER_BLOCK_MAX) wf_bounce(J jobs, WfBuffers B, WfIter w, unsigned long long* counters,
-                                                 uint32_t* status_word) {
+// Several iterations in one launch: each queued slot runs `steps` bounces (trace, then wf_step) on its own
+// thread, and the slots still live go to the next queue.  The slots do not wait for one another between
+// bounces, so a batch of iterations over a queue that no longer fills the GPU costs one launch instead of
+// two a bounce, each with its ramp and its tail; over a long queue the split kernels win (64 registers
+// against this one's 96, and no lanes that wait for other lanes' materials).  A step goes through the slot's
+// record exactly as the split kernels' does - the same arithmetic in the same order - so where a bounce runs
+// does not change it.  Rule (run_wavefront): at most 2,048 queued slots per SM.  Measured at 1,024 / 2,048 /
+// 4,096 slots per SM against the split kernels only: spheres 1280x720 55.5 / 54.9 / 55.2 against 56.8 ms,
+// meshes (1.31 M triangles) 62.9 / 62.3 / 62.3 against 64.1, transforms 333x251 7.00 / 6.90 / 6.91 against
+// 7.24; Cornell 256x256 1.60 against 1.79, 64x48 preview 0.26 against 0.44 ms.  96 registers (20 warps per
+// SM) beat 128: spheres 54.9 against 55.9 ms.
+template <bool CLEAN, int ORDER, class J>
+__global__ void __launch_bounds__(WF_BOUNCES_BLOCK, 20) wf_bounces(J jobs, WfBuffers B, WfIter w, int steps,
+                                                                   uint32_t* status_word) {
     const uint32_t n = B.ctr[w.cin];
     if (blockIdx.x == 0 && threadIdx.x == 0) B.ctr[w.czero] = 0u;   // appended to by the next iteration
     const WfWindow win = jobs.window();
     const uint32_t* q = B.queue[w.qin];
-    uint32_t* qn = B.queue[w.qin ^ 1];
-    uint32_t* cn = B.ctr + w.cout;
-    uint32_t status = 0, paths = 0, rays = 0;
+    uint32_t status = 0, paths = 0;
     PathCounters pc{0, 0, 0};
     TraceStats st{0, 0};
-    const uint32_t stride = gridDim.x * blockDim.x;
-    const uint32_t limit = (n + 31u) & ~31u;
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < limit; k += stride) {
-        bool live = false;
+    const uint32_t stride = gridDim.x * WF_BOUNCES_BLOCK;
+    for (uint32_t base = blockIdx.x * WF_BOUNCES_BLOCK; base < n; base += stride) {   // whole warps
+        const uint32_t k = base + threadIdx.x;
+        bool live = k < n;
         uint32_t slot = 0;
-        if (k < n) {
-            slot = ld_state(q + k);
-            const Sec R = ld_sec(wf_sec(B, slot, SEC_RAY));
-            const Sec SH = ld_sec(wf_sec(B, slot, SEC_SHADE));
-            const Sec PX = ld_sec(wf_sec(B, slot, SEC_PIXEL));
-            const uint32_t mw = R.w[7];
-            const uint32_t job = wf_job(mw);
-            float t;
-            uint32_t item;
-            ++rays;
-            bool h = closest_hit<CLEAN>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), wf_tmin(sec_f(R, 6)), 3.402823466e+38f,
-                                        wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t, item, st, status);
-            live = wf_step<CLEAN, ORDER>(jobs, win, B, slot, R, SH, PX, t, h ? item : 0xffffffffu, pc, st, paths, status);
+        if (live) slot = ld_state(q + k);
+        for (int s = 0; s < steps && __any_sync(0xffffffffu, live); ++s) {
+            if (live) {
+                const Sec R = ld_sec<true>(wf_sec(B, slot, SEC_RAY));
+                const Sec SH = ld_sec<true>(wf_sec(B, slot, SEC_SHADE));
+                const Sec PX = ld_sec<true>(wf_sec(B, slot, SEC_PIXEL));
+                const uint32_t mw = R.w[7];
+                const uint32_t job = wf_job(mw);
+                float t;
+                uint32_t item;
+                const bool h = closest_hit<CLEAN>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), wf_tmin(sec_f(R, 6)),
+                                                  3.402823466e+38f, wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t,
+                                                  item, st, status);
+                live = wf_step<CLEAN, ORDER, true>(jobs, win, B, slot, R, SH, PX, t, h ? item : 0xffffffffu, pc, st, paths,
+                                                   status);
+            }
         }
-        wf_push(qn, cn, slot, live);
+        wf_push(B.queue[w.qin ^ 1], B.ctr + w.cout, slot, live);
     }
-    wf_flush<COUNT>(counters, rays + pc.rays, paths, st);
     if (status) atomicOr(status_word, status);
 }
 
@@ -1029,9 +1047,11 @@ cudaError_t wf_dispatch(WfOp op, const A& args, const WfBuffers& B, const WfLaun
     case WF_OP_SPLIT:
         wf_split<CLEAN><<<L.grid, 128, 0, L.st>>>(jobs, B, L.w, L.k0, L.threshold);
         break;
-    case WF_OP_BOUNCE:
-        if (c) wf_bounce<CLEAN, ORDER, true><<<L.grid, blk, 0, L.st>>>(jobs, B, L.w, L.counters, L.status);
-        else wf_bounce<CLEAN, ORDER, false><<<L.grid, blk, 0, L.st>>>(jobs, B, L.w, nullptr, L.status);
+    case WF_OP_BOUNCES:
+        // one image only: a ring's slots take new pixels at every iteration
+        if constexpr (std::is_same<J, WfOne>::value)
+            wf_bounces<CLEAN, ORDER><<<L.grid, WF_BOUNCES_BLOCK, 0, L.st>>>(jobs, B, L.w, L.steps, L.status);
+        else return cudaErrorInvalidValue;
         break;
     default:
         return cudaErrorInvalidValue;
