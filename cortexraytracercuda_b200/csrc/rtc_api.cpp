@@ -1139,7 +1139,6 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     cudaError_t e = fn(WF_OP_INIT, J, B, L);
     if (e != cudaSuccess) return cuda_fail(e, "wavefront init");
     run.launches = 1;
-    L.grid = grid;
     const uint64_t nsamp = clean ? (uint64_t)P.spp : (uint64_t)P.sqrt_spp * P.sqrt_spp;
     const uint64_t rounds = (uint64_t)((P.num_pixels * P.groups + B.slots - 1) / B.slots);
     const uint64_t max_iters = rounds * nsamp * (uint64_t)(P.max_depth + 1) + 64;
@@ -1152,12 +1151,17 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     // make a bounce instruction-bound, where packing pays (5-15% of a frame at 16 or more spp); elsewhere
     // the longest chains' latency bounds the drain and repacking costs 2-50% (wf_finish, wf_finish_packed).
     L.drain_every = rtc_drain_every(S.num_xnodes ? 2 : 0);
-    // Queue chunks handed out by a counter for scenes of 2^20 primitives or more, whose walks are long
-    // and uneven (meshes frame, 1.31 M triangles: extend 450.7 -> 405.5 ms, 436 -> 460-467 Mpaths/s);
-    // the fixed grid stride for smaller ones (spheres frame, 489 primitives: 945 against 840 Mpaths/s;
-    // the 64 batch scenes of up to 500 K triangles, one image per call: 631 against 608 in compat mode,
-    // 1,167 against 1,001 in clean mode with sample groups).
-    L.dynamic = rtc_dynamic_chunks(S.num_items >= (1u << 20));
+    // Work distribution of the iteration kernels.  Extend: one 32-entry chunk per warp, the grid as long as
+    // the queue can be, so that the block scheduler balances uneven walks and no launch ends on the stride's
+    // last, half-empty round (8 blocks per SM striding the queue: spheres frame 54.7 against 53.7 ms, a
+    // 20,480-triangle frame with the 8-wide nodes 15.2 against 14.4).  From 2^20 primitives on, chunks handed out by a counter to
+    // 8 blocks per SM, whose warps keep their place in the caches (1.31 M triangles: extend 49.8 ms against
+    // 50.2 with the long grid and 53.8 with the stride).  Shade: 8 blocks per SM striding the queue (one
+    // resident wave; the long grid costs it 5-15%); the counter costs it more than it balances (same frame: 10.1
+    // against 8.3 ms), but clean mode keeps it in those scenes, where the two kernels round a refraction
+    // differently in the last bit.
+    const bool large = S.num_items >= (1u << 20);
+    const bool dynamic_extend = rtc_dynamic_chunks(large), dynamic_shade = rtc_dynamic_chunks(large && clean);
     // long-chain split: at iteration `split_at` (0: never), slots predicted to need more than
     // `split_thr` further iterations move to the drain kernel, running beside the bulk iterations
     uint64_t split_at = 0;
@@ -1168,8 +1172,9 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     if (const char* ev = std::getenv("RTC_WF_SPLIT_BLOCKS")) split_blocks = std::max(1, std::atoi(ev));
     int64_t last_left = -1;   // queue size last observed (one batch late in both polling modes)
     // A batch of iterations over at most this many queued slots is one wf_bounces launch (see there); the
-    // instrumented and the timed forms and the 8-wide walk keep the split kernels.
-    uint32_t bounces_max = timer || d_counters || L.wide ? 0u : (uint32_t)num_sms * 2048u;
+    // instrumented and the timed forms and the 8-wide walk keep the split kernels, and so do frames shaded
+    // with dynamic chunks (see above: their last bits).
+    uint32_t bounces_max = timer || d_counters || L.wide || dynamic_shade ? 0u : (uint32_t)num_sms * 2048u;
     if (const char* ev = std::getenv("RTC_WF_BOUNCES")) bounces_max = std::min(bounces_max, (uint32_t)std::strtoul(ev, nullptr, 10));
     const int64_t units = P.num_pixels * P.groups;
     uint64_t rot = 0;   // queue rotations: one per launch that reads one queue and fills the other
@@ -1208,6 +1213,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
             L.w = wf_iter(rot++);
             L.k0 = (float)it;
             L.threshold = split_thr;
+            L.grid = grid;
             e = fn(WF_OP_SPLIT, J, B, L);
             if (e != cudaSuccess) return cuda_fail(e, "wavefront split");
             ++it;
@@ -1226,20 +1232,25 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
             if (e != cudaSuccess) return cuda_fail(e, "wavefront long chains");
             if (poll.st_long) RTC_CUDA(cudaEventRecord(poll.split_ev[1], poll.st_long));
         }
-        // the queue only shrinks while the units fit the slots (a finished unit's slot has none to take)
-        const int64_t bound = last_left >= 0 ? last_left : units;
-        if (units <= (int64_t)B.slots && bound <= (int64_t)bounces_max) {
+        // what the queue can hold: while the units fit the slots it only shrinks (a finished unit's slot has
+        // none to take)
+        const bool shrinks = units <= (int64_t)B.slots;
+        const int64_t bound = !shrinks ? (int64_t)B.slots : last_left >= 0 ? last_left : units;
+        const bool bounces = shrinks && bound <= (int64_t)bounces_max;
+        if (bounces) {
             L.w = wf_iter(rot++);
             L.steps = BATCH;
             L.grid = (int)std::max<int64_t>(1, (bound + rtc::WF_BOUNCES_BLOCK - 1) / rtc::WF_BOUNCES_BLOCK);
             e = fn(WF_OP_BOUNCES, J, B, L);
-            L.grid = grid;
             if (e != cudaSuccess) return cuda_fail(e, "wavefront iterations");
             it += BATCH;
             ++run.launches;
         } else {
+            const int long_grid = (int)std::max<int64_t>(1, (bound + 127) / 128);   // 128-thread blocks
             for (int k = 0; k < BATCH; ++k, ++it) {
                 L.w = wf_iter(rot++);
+                L.dynamic = dynamic_extend;
+                L.grid = dynamic_extend ? grid : long_grid;
                 cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr, e3 = nullptr;
                 if (timer) {
                     RTC_CUDA(timer->pair(e0, e1));
@@ -1252,6 +1263,8 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
                     RTC_CUDA(cudaEventRecord(e2, st));
                     timer->ext.push_back({e0, e1});
                 }
+                L.dynamic = dynamic_shade;
+                L.grid = std::min(long_grid, grid);
                 if (e == cudaSuccess) e = fn(WF_OP_SHADE, J, B, L);
                 if (timer) {
                     RTC_CUDA(cudaEventRecord(e3, st));
@@ -1263,7 +1276,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
         }
         // A frame of fewer units than the drain threshold always drains after its second batch (the count of
         // the first is at most the units): nothing to wait for.
-        if (bound <= (int64_t)bounces_max && units <= (int64_t)B.slots && units < (int64_t)drain && split_at == 0) {
+        if (bounces && units < (int64_t)drain && split_at == 0) {
             if (b == 0) continue;
             left = (uint32_t)units;
             run.drained = true;
