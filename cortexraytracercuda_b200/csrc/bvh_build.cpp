@@ -5,8 +5,11 @@
 #include <atomic>
 #include <cfloat>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <tuple>
 
@@ -42,114 +45,142 @@ inline double area(const Aabb& a) {
     return 2.0 * (dx * dy + dy * dz + dz * dx);
 }
 
-constexpr int PAR_DEPTH = 4;            // subtrees below the first four levels are built concurrently
-constexpr uint32_t PAR_MIN = 32768;     // ... when they hold at least this many primitives
+constexpr int PAR_DEPTH = 6;            // subtrees below the first six levels are built concurrently
+constexpr uint32_t PAR_MIN = 4096;      // ... when they hold at least this many primitives
+constexpr uint32_t SMALL_NODE = 16;     // nodes of at most this many primitives are split without bin tables
 
-struct Shared {
-    const std::vector<Aabb>& boxes;
-    std::vector<float> cen;          // 3 per primitive
-    std::vector<uint32_t> idx;       // subtrees partition disjoint ranges of it
-    int max_leaf;
+// A primitive under construction: its box and centroid travel with it when nodes are partitioned, so a
+// node's passes read memory in order.
+struct Prim {
+    Aabb box;
+    float cen[3];
+    uint32_t id;
 };
 
+// Nodes live in one array: a subtree of m primitives has at most 2 m - 1 nodes, so the one that starts at
+// `id` owns ids [id, id + 2 m - 1) and its halves can be built anywhere in that range at the same time.
 struct Builder {
-    Shared& sh;
-    const std::vector<Aabb>& boxes;
-    std::vector<float>& cen;
-    std::vector<uint32_t>& idx;
-    int max_leaf;
-    std::vector<BNode> nodes;        // per-builder (one per subtree task)
+    Prim* const prims;               // subtrees partition disjoint ranges
+    BNode* const nodes;
+    const int max_leaf;
 
-    explicit Builder(Shared& s) : sh(s), boxes(s.boxes), cen(s.cen), idx(s.idx), max_leaf(s.max_leaf) {}
+    struct Split {
+        int axis = -1, bin = -1;
+        double cost = DBL_MAX;
+    };
 
-    // Appends another builder's tree (its node 0 is its root); returns the root's id here.
-    int32_t splice(const Builder& o) {
-        const int32_t off = (int32_t)nodes.size();
-        for (BNode b : o.nodes) {
-            if (!b.leaf) {
-                b.left += off;
-                b.right += off;
-            }
-            nodes.push_back(b);
-        }
-        return off;
+    static int bin_of(float c, float lo, double scale) {
+        const int b = (int)(((double)c - lo) * scale);
+        return b < 0 ? 0 : (b >= NBINS ? NBINS - 1 : b);
     }
 
-    int32_t build(uint32_t start, uint32_t end, int depth, uint32_t& max_depth) {
-        int32_t id = (int32_t)nodes.size();
-        nodes.emplace_back();
+    // Best binned SAH split of [start, end) along one axis, over a table of all the bins.
+    void split_binned(uint32_t start, uint32_t end, int ax, float lo, double scale, double parea, Split& best) const {
+        uint32_t cnt[NBINS] = {0};
+        Aabb bb[NBINS];
+        for (int b = 0; b < NBINS; ++b) bb[b] = empty_box();
+        for (uint32_t i = start; i < end; ++i) {
+            const int b = bin_of(prims[i].cen[ax], lo, scale);
+            cnt[b]++;
+            grow(bb[b], prims[i].box);
+        }
+        double la[NBINS];
+        uint32_t lc[NBINS];
+        Aabb acc = empty_box();
+        uint32_t c = 0;
+        for (int b = 0; b < NBINS - 1; ++b) {
+            if (cnt[b]) grow(acc, bb[b]);
+            c += cnt[b];
+            la[b] = cnt[b] || b == 0 ? area(acc) : la[b - 1];
+            lc[b] = c;
+        }
+        acc = empty_box();
+        c = 0;
+        for (int b = NBINS - 1; b > 0; --b) {
+            if (!cnt[b]) continue;   // the same halves as the split just tried: never strictly cheaper
+            grow(acc, bb[b]);
+            c += cnt[b];
+            const uint32_t nl = lc[b - 1];
+            if (nl == 0) continue;
+            const double cost = 1.0 + (la[b - 1] * nl + area(acc) * c) / parea;
+            if (cost < best.cost) best = {ax, b, cost};
+        }
+    }
+
+    // The same split of a small node: its few primitives in bin order take the place of the table (boxes
+    // grow by min and max, so the order within a bin does not matter).
+    void split_small(uint32_t start, uint32_t end, int ax, float lo, double scale, double parea, Split& best) const {
+        const int n = (int)(end - start);
+        int bin[SMALL_NODE];
+        const Aabb* box[SMALL_NODE];
+        for (int i = 0; i < n; ++i) {
+            const Prim& p = prims[start + (uint32_t)i];
+            const int b = bin_of(p.cen[ax], lo, scale);
+            int j = i;
+            for (; j > 0 && bin[j - 1] > b; --j) {
+                bin[j] = bin[j - 1];
+                box[j] = box[j - 1];
+            }
+            bin[j] = b;
+            box[j] = &p.box;
+        }
+        double la[SMALL_NODE];   // area of the primitives before i, where i starts a bin
+        Aabb acc = empty_box();
+        for (int i = 0; i < n; ++i) {
+            if (i && bin[i] != bin[i - 1]) la[i] = area(acc);
+            grow(acc, *box[i]);
+        }
+        acc = empty_box();
+        for (int i = n - 1; i > 0; --i) {
+            grow(acc, *box[i]);
+            if (bin[i] == bin[i - 1]) continue;
+            const double cost = 1.0 + (la[i] * (uint32_t)i + area(acc) * (uint32_t)(n - i)) / parea;
+            if (cost < best.cost) best = {ax, bin[i], cost};
+        }
+    }
+
+    void build(uint32_t start, uint32_t end, int32_t id, int depth, uint32_t& max_depth) const {
+        BNode& node = nodes[id];
+        node = BNode{};
         Aabb box = empty_box(), cb = empty_box();
         for (uint32_t i = start; i < end; ++i) {
-            uint32_t p = idx[i];
-            grow(box, boxes[p]);
+            const Prim& p = prims[i];
+            grow(box, p.box);
             for (int k = 0; k < 3; ++k) {
-                cb.lo[k] = std::min(cb.lo[k], cen[3 * p + k]);
-                cb.hi[k] = std::max(cb.hi[k], cen[3 * p + k]);
+                cb.lo[k] = std::min(cb.lo[k], p.cen[k]);
+                cb.hi[k] = std::max(cb.hi[k], p.cen[k]);
             }
         }
-        nodes[id].box = box;
+        node.box = box;
         if ((uint32_t)depth > max_depth) max_depth = depth;
         const uint32_t n = end - start;
         auto make_leaf = [&]() {
-            nodes[id].leaf = true;
-            nodes[id].first = start;
-            nodes[id].count = n;
-            return id;
+            node.leaf = true;
+            node.first = start;
+            node.count = n;
         };
-        if (n <= 1) return make_leaf();
+        if (n <= 1) { make_leaf(); return; }
 
         // best binned SAH split
-        int best_axis = -1, best_bin = -1;
-        double best_cost = DBL_MAX;
+        Split best;
         const double parea = std::max(area(box), 1e-30);
         for (int ax = 0; ax < 3; ++ax) {
-            double ext = (double)cb.hi[ax] - cb.lo[ax];
+            const double ext = (double)cb.hi[ax] - cb.lo[ax];
             if (!(ext > 0.0)) continue;
-            uint32_t cnt[NBINS] = {0};
-            Aabb bb[NBINS];
-            for (int b = 0; b < NBINS; ++b) bb[b] = empty_box();
-            const double scale = NBINS / ext;
-            for (uint32_t i = start; i < end; ++i) {
-                uint32_t p = idx[i];
-                int b = (int)(((double)cen[3 * p + ax] - cb.lo[ax]) * scale);
-                b = b < 0 ? 0 : (b >= NBINS ? NBINS - 1 : b);
-                cnt[b]++;
-                grow(bb[b], boxes[p]);
-            }
-            double la[NBINS];
-            uint32_t lc[NBINS];
-            Aabb acc = empty_box();
-            uint32_t c = 0;
-            for (int b = 0; b < NBINS - 1; ++b) {
-                grow(acc, bb[b]);
-                c += cnt[b];
-                la[b] = area(acc);
-                lc[b] = c;
-            }
-            acc = empty_box();
-            c = 0;
-            for (int b = NBINS - 1; b > 0; --b) {
-                grow(acc, bb[b]);
-                c += cnt[b];
-                uint32_t nl = lc[b - 1];
-                if (nl == 0 || c == 0) continue;
-                double cost = 1.0 + (la[b - 1] * nl + area(acc) * c) / parea;
-                if (cost < best_cost) { best_cost = cost; best_axis = ax; best_bin = b; }
-            }
+            if (n <= SMALL_NODE) split_small(start, end, ax, cb.lo[ax], NBINS / ext, parea, best);
+            else split_binned(start, end, ax, cb.lo[ax], NBINS / ext, parea, best);
         }
         const bool can_leaf = n <= (uint32_t)max_leaf;
-        if (can_leaf && (best_axis < 0 || (double)n <= best_cost)) return make_leaf();
+        if (can_leaf && (best.axis < 0 || (double)n <= best.cost)) { make_leaf(); return; }
 
         uint32_t mid;
-        if (best_axis >= 0 && depth < MAX_TREE_DEPTH) {
-            const double ext = (double)cb.hi[best_axis] - cb.lo[best_axis];
+        if (best.axis >= 0 && depth < MAX_TREE_DEPTH) {
+            const double ext = (double)cb.hi[best.axis] - cb.lo[best.axis];
             const double scale = NBINS / ext;
-            auto it = std::partition(idx.begin() + start, idx.begin() + end, [&](uint32_t p) {
-                int b = (int)(((double)cen[3 * p + best_axis] - cb.lo[best_axis]) * scale);
-                b = b < 0 ? 0 : (b >= NBINS ? NBINS - 1 : b);
-                return b < best_bin;
+            Prim* it = std::partition(prims + start, prims + end, [&](const Prim& p) {
+                return bin_of(p.cen[best.axis], cb.lo[best.axis], scale) < best.bin;
             });
-            mid = (uint32_t)(it - idx.begin());
+            mid = (uint32_t)(it - prims);
             if (mid == start || mid == end) mid = start + n / 2;
         } else {
             // median split on the widest centroid axis (also the fallback for coincident centroids)
@@ -157,54 +188,56 @@ struct Builder {
             for (int k = 1; k < 3; ++k)
                 if (cb.hi[k] - cb.lo[k] > cb.hi[ax] - cb.lo[ax]) ax = k;
             mid = start + n / 2;
-            std::nth_element(idx.begin() + start, idx.begin() + mid, idx.begin() + end,
-                             [&](uint32_t a, uint32_t b) { return cen[3 * a + ax] < cen[3 * b + ax]; });
+            std::nth_element(prims + start, prims + mid, prims + end,
+                             [&](const Prim& a, const Prim& b) { return a.cen[ax] < b.cen[ax]; });
         }
-        if (depth <= PAR_DEPTH && n >= PAR_MIN) {
-            // the two halves on two threads, each into its own node array, then spliced in
-            Builder L(sh), R(sh);
+        node.left = id + 1;
+        node.right = id + 2 * (int32_t)(mid - start);
+        if (depth <= PAR_DEPTH && n >= PAR_MIN) {   // the two halves on two threads
             uint32_t dl = 0, dr = 0;
-            std::thread t([&] { L.build(start, mid, depth + 1, dl); });
-            R.build(mid, end, depth + 1, dr);
-            t.join();
+            std::thread t;
+            try {
+                t = std::thread([&] { build(start, mid, node.left, depth + 1, dl); });
+            } catch (const std::system_error&) {   // no thread to be had: this one does both
+                build(start, mid, node.left, depth + 1, dl);
+            }
+            build(mid, end, node.right, depth + 1, dr);
+            if (t.joinable()) t.join();
             max_depth = std::max(max_depth, std::max(dl, dr));
-            const int32_t l = splice(L);
-            const int32_t r = splice(R);
-            nodes[id].left = l;
-            nodes[id].right = r;
-            return id;
+            return;
         }
-        int32_t l = build(start, mid, depth + 1, max_depth);
-        int32_t r = build(mid, end, depth + 1, max_depth);
-        nodes[id].left = l;
-        nodes[id].right = r;
-        return id;
+        build(start, mid, node.left, depth + 1, max_depth);
+        build(mid, end, node.right, depth + 1, max_depth);
     }
 };
 
 }  // namespace
 
-bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, const char** err) {
+bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, const char** err, bool wide) {
     (void)threads;
     const size_t n = in.boxes.size();
     if (max_leaf < 1) max_leaf = 1;
     if (max_leaf > MAX_LEAF) max_leaf = MAX_LEAF;
     if (n >= (1u << 26)) { if (err) *err = "too many primitives for the leaf encoding (max 2^26)"; return false; }
-    Shared SH{in.boxes, {}, {}, max_leaf};
-    SH.cen.resize(3 * n);
-    SH.idx.resize(n);
+    // uninitialised: every record is written by the pass that makes it
+    std::unique_ptr<Prim[]> prims(new Prim[std::max<size_t>(n, 1)]);
+    std::unique_ptr<BNode, void (*)(void*)> node_mem((BNode*)std::malloc(sizeof(BNode) * std::max<size_t>(2 * n, 1)), std::free);
+    if (!node_mem) { if (err) *err = "host allocation failed"; return false; }
     for (size_t p = 0; p < n; ++p) {
-        SH.idx[p] = (uint32_t)p;
-        for (int k = 0; k < 3; ++k) SH.cen[3 * p + k] = 0.5f * (in.boxes[p].lo[k] + in.boxes[p].hi[k]);
+        prims[p].box = in.boxes[p];
+        prims[p].id = (uint32_t)p;
+        for (int k = 0; k < 3; ++k) prims[p].cen[k] = 0.5f * (in.boxes[p].lo[k] + in.boxes[p].hi[k]);
     }
-    Builder B(SH);
-    B.nodes.reserve(2 * n + 2);
+    const Builder B{prims.get(), node_mem.get(), max_leaf};
     uint32_t max_depth = 0;
-    int32_t root = n ? B.build(0, (uint32_t)n, 1, max_depth) : -1;
+    const int32_t root = n ? 0 : -1;
+    if (n) B.build(0, (uint32_t)n, root, 1, max_depth);
 
     // Flatten: inner nodes in depth-first order, leaves folded into their parent's child slots.
     out.nodes.clear();
+    out.nodes.reserve(16 * std::max<size_t>(n, 1));
     out.order.clear();
+    out.order.reserve(n);
     out.max_leaf_seen = 0;
     std::vector<int32_t> stack;
     auto alloc_node = [&]() {
@@ -213,7 +246,7 @@ bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, co
     };
     auto encode_leaf = [&](const BNode& L) -> int32_t {
         uint32_t first = (uint32_t)out.order.size();
-        for (uint32_t i = 0; i < L.count; ++i) out.order.push_back(B.idx[L.first + i]);
+        for (uint32_t i = 0; i < L.count; ++i) out.order.push_back(prims[L.first + i].id);
         if (L.count > out.max_leaf_seen) out.max_leaf_seen = L.count;
         return (int32_t)~((first << LEAF_COUNT_BITS) | L.count);
     };
@@ -280,13 +313,16 @@ bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, co
     //    quantised test never loses a hit the binary nodes find.
     out.nodes8.clear();
     out.items8.clear();
+    out.num_nodes8 = 0;
+    if (max_depth + 2 > (uint32_t)TRAVERSAL_STACK) { if (err) *err = "BVH too deep for the traversal stack"; return false; }
+    if (!wide) return true;
     auto alloc8 = [&](int count) {
         const int32_t first = (int32_t)(out.nodes8.size() / NODE8_FLOATS);
         out.nodes8.resize(out.nodes8.size() + (size_t)count * NODE8_FLOATS, 0.0f);
         return first;
     };
     // the binary flattening's leaf encoding of each binary leaf (replayed in its DFS left-first order)
-    std::vector<int32_t> leaf_of(B.nodes.size(), 0);
+    std::vector<int32_t> leaf_of(2 * n, 0);
     {
         std::vector<int32_t> st;
         if (root >= 0) st.push_back(root);
@@ -367,7 +403,8 @@ bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, co
         uint8_t q[3][2][8] = {};   // axis, (low, high), slot
         for (int k = 0; k < 3; ++k) {
             const double ext = (double)nb.hi[k] - (double)nb.lo[k];
-            int e = -126;
+            // the least e >= -126 with 255 * 2^e >= ext, counted up from 255 * 2^(exponent of ext - 9) < ext
+            int e = ext > 0.0 ? std::min(std::max(std::ilogb(ext) - 9, -126), 127) : -126;
             while (e < 127 && std::ldexp(255.0, e) < ext) ++e;
             const double step = std::ldexp(1.0, e);
             hdr |= (uint32_t)(e + 127) << (8 * k);
@@ -440,7 +477,6 @@ bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, co
         out.items8.clear();
         out.num_nodes8 = 0;
     }
-    if (max_depth + 2 > (uint32_t)TRAVERSAL_STACK) { if (err) *err = "BVH too deep for the traversal stack"; return false; }
     return true;
 }
 

@@ -34,7 +34,8 @@ struct BvhOutput {
 };
 
 // Returns false (with a message) if the tree would not fit the traversal stack or the item encoding.
-bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, const char** err);
+// `wide`: also make the 8-wide nodes.
+bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, const char** err, bool wide = true);
 
 // Merges subtrees of at most `max_leaf` primitives into single leaves where the SAH cost favours it
 // (bvh_build.cpp): renumbers the nodes depth-first and reorders `order` so each leaf is contiguous;

@@ -340,7 +340,7 @@ bool join_top(const std::vector<Cluster>& rest, std::vector<float>& nodes, const
     for (size_t i = 0; i < rest.size(); ++i) tin.boxes[i] = rest[i].box;
     BvhOutput top;
     const char* terr = nullptr;
-    if (!build_bvh(tin, 1, 0, top, &terr) || top.num_nodes != rest.size() - 1) {
+    if (!build_bvh(tin, 1, 0, top, &terr, false) || top.num_nodes != rest.size() - 1) {
         *what = terr ? terr : "device BVH build: the top-level join failed";
         return false;
     }

@@ -513,13 +513,19 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     std::vector<uint32_t> main_ids, x_ids;
     BvhInput bin_x;
     {
-        BvhInput bin_main;
-        for (uint32_t i = 0; i < (uint32_t)prims.size(); ++i) {
-            const bool x = prims[i].kind == ITEM_XPRIM;
-            (x ? x_ids : main_ids).push_back(i);
-            (x ? bin_x : bin_main).boxes.push_back(bin.boxes[i]);
+        size_t nx = 0;
+        for (const PrimRef& p : prims) nx += p.kind == ITEM_XPRIM;
+        main_ids.reserve(prims.size() - nx);
+        x_ids.reserve(nx);
+        for (uint32_t i = 0; i < (uint32_t)prims.size(); ++i) (prims[i].kind == ITEM_XPRIM ? x_ids : main_ids).push_back(i);
+        if (nx) {
+            BvhInput bin_main;
+            bin_main.boxes.reserve(main_ids.size());
+            bin_x.boxes.reserve(nx);
+            for (uint32_t i : main_ids) bin_main.boxes.push_back(bin.boxes[i]);
+            for (uint32_t i : x_ids) bin_x.boxes.push_back(bin.boxes[i]);
+            bin = std::move(bin_main);
         }
-        bin = std::move(bin_main);
     }
     BvhOutput bvh, xbvh;
     const char* berr = nullptr;
@@ -592,6 +598,11 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     for (uint32_t m = 0; m < d->num_meshes; ++m) any_uv = any_uv || d->meshes[m].uvs != nullptr;
     std::vector<int2> sph_aux;
     std::vector<int4> xprim;
+    sph.reserve(d->num_spheres);
+    sph_aux.reserve(d->num_spheres);
+    tri.reserve(3 * ntri);
+    tri_n.reserve(ntri);
+    if (any_uv) tri_uv.reserve(2 * ntri);
     // global id bases: the lights come first, in light-list order (index = light id = global id); one id
     // per box
     const uint32_t base_sph = nlights, base_quad = base_sph + d->num_spheres, base_box = base_quad + d->num_quads,
@@ -796,9 +807,14 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     size_t o_envcdf = add_chunk(env_cdf.data(), env_cdf.size() * sizeof(float));
 
     // host image of the device slab; the DevScene's pointer fields hold byte offsets into it
-    H.slab.assign(total, 0);
-    for (const Chunk& c : chunks)
-        if (c.src && c.bytes) std::memcpy(H.slab.data() + c.off, c.src, c.bytes);
+    if (!H.slab.make(total)) return fail(RTC_ERR_OOM, "host allocation failed");
+    for (size_t i = 0; i < chunks.size(); ++i) {
+        const Chunk& c = chunks[i];
+        const size_t end = i + 1 < chunks.size() ? chunks[i + 1].off : total;
+        const size_t used = c.src ? c.bytes : 0;
+        if (used) std::memcpy(H.slab.data() + c.off, c.src, used);
+        std::memset(H.slab.data() + c.off + used, 0, end - c.off - used);   // padding
+    }
     auto off = [](size_t o) { return reinterpret_cast<uint8_t*>(static_cast<uintptr_t>(o)); };
     DevScene& D = H.dev;
     D = DevScene{};

@@ -5,6 +5,7 @@
 
 #include <memory>
 #include <mutex>
+#include <new>
 #include <utility>
 #include <vector>
 
@@ -54,11 +55,28 @@ struct rtc_scene {
 };
 
 
+// Host memory that is not cleared when it is made (its maker writes every byte that is read).
+class Slab {
+public:
+    bool make(size_t bytes) {
+        mem_.reset(new (std::nothrow) uint8_t[bytes]);
+        size_ = mem_ ? bytes : 0;
+        return mem_ != nullptr;
+    }
+    uint8_t* data() { return mem_.get(); }
+    const uint8_t* data() const { return mem_.get(); }
+    size_t size() const { return size_; }
+
+private:
+    std::unique_ptr<uint8_t[]> mem_;
+    size_t size_ = 0;
+};
+
 // Host image of a scene: the flattened device slab (BVH, primitives, materials, textures, images,
 // environment map) built once on the host, uploadable to any device address.  Pointer fields of `dev`
 // hold byte offsets into `slab`.
 struct HostScene {
-    std::vector<uint8_t> slab;
+    Slab slab;
     rtc::DevScene dev{};
     rtc_camera cam{};
     rtc_scene_info info{};
