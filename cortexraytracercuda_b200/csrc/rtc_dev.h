@@ -163,25 +163,30 @@ struct DevParams {
 
 // Wavefront path slots (one slot = one pixel, or one sample group, in flight) and the slot queues.
 //
-// A slot's path state is one 96-byte record of three 32-byte sectors, each moved by a single 256-bit
-// load or store (the kernels reach slots through the queues, so neighbouring lanes touch unrelated
-// records: a sector per access is the least a scattered access can move):
-//   sector 0, ray:    origin.xyz, direction.xyz, the trace's start (0 for an ordinary ray, t + 0.001 for
-//                     the re-hit from behind a one-sided light, camera.cuh:177-183), and the depth word
-//                     (depth left in the low 16 bits | job slot in the high 16 bits, 0 for one image);
+// A slot's path state is three 32-byte sectors, each moved by a single 256-bit load or store (the kernels
+// reach slots through the queues, so neighbouring lanes touch unrelated records: a sector per access is the
+// least a scattered access can move).  The first two, which every bounce moves, lie together in `rec`; the
+// third has an array of its own, so that what a bounce touches is dense in L2:
+//   sector 0, ray:    origin.xyz, direction.xyz; compat: the pixel's minstd state (31 bits) and in the top
+//                     bit whether the ray is the re-hit from behind a one-sided light (camera.cuh:177-183);
+//                     clean: the trace's start (0 for an ordinary ray, t + 0.001 for the re-hit); and the
+//                     depth word (depth left in the low 16 bits | job slot in the high 16 bits, 0 for one
+//                     image);
 //   sector 1, shade:  path attenuation rgb, radiance of the current sample rgb, and the closest hit the
-//                     extend kernel found (t, item bits; 0xffffffff = miss);
-//   sector 2, pixel:  pixel (0xffffffff = idle slot), sample index, the minstd state (compat) or the
-//                     sample group (clean), the PCG32 state's low word (clean), the pixel sum rgb, and
-//                     the PCG32 state's high word.  A clean-mode stream's increment is 2 s + 1 for sample
-//                     s (Pcg32::seed), so it is recomputed from the sample index, not stored.
+//                     extend kernel found (t, item bits; 0xffffffff = miss); a compat re-hit waits here
+//                     with its start in place of t;
+//   sector 2, pixel:  pixel (0xffffffff = idle slot), sample index, the sample group, the PCG32 state's
+//                     low word (clean), the pixel sum rgb, and the PCG32 state's high word.  A clean-mode
+//                     stream's increment is 2 s + 1 for sample s (Pcg32::seed), so it is recomputed from the
+//                     sample index, not stored.  Compat mode touches it only where a sample ends.
 // The ray's time (perspective_camera::get_ray draws it) is not kept: no hit test reads it.
-constexpr uint32_t WF_REC_WORDS = 24;
-constexpr uint32_t WF_REC_BYTES = WF_REC_WORDS * 4;
+constexpr uint32_t WF_REC_WORDS = 16;   // sectors 0 and 1
+constexpr uint32_t WF_PX_WORDS = 8;     // sector 2
 struct WfBuffers {
     uint32_t* rec;        // slots x WF_REC_WORDS words, 256-byte aligned (so every sector is 32-byte aligned)
+    uint32_t* px;         // slots x WF_PX_WORDS words, likewise
     uint32_t* queue[3];   // [0], [1]: the alternating slot queues; [2]: slots split off as long chains
-    uint32_t* ctr;        // [0..2] queue sizes (rotating), [3] next pixel to fetch, [4] long-chain queue size
+    uint32_t* ctr;        // WfCtr: [0..2] queue sizes (rotating), next pixel, long chains, chunk counters
     uint32_t slots;
 };
 

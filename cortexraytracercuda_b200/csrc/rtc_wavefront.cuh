@@ -71,7 +71,7 @@ __device__ __forceinline__ T ld_state(const T* p) {
 #endif
 }
 
-// ---- slot records (WfBuffers::rec): three 32-byte sectors per slot, one 256-bit access each --------
+// ---- slot records (WfBuffers::rec, px): three 32-byte sectors per slot, one 256-bit access each ----
 
 struct Sec {
     uint32_t w[8];
@@ -79,7 +79,7 @@ struct Sec {
 constexpr int SEC_RAY = 0, SEC_SHADE = 1, SEC_PIXEL = 2;
 
 __device__ __forceinline__ uint32_t* wf_sec(const WfBuffers& B, uint32_t slot, int sec) {
-    return B.rec + (size_t)slot * WF_REC_WORDS + 8 * sec;
+    return sec == SEC_PIXEL ? B.px + 8 * (size_t)slot : B.rec + WF_REC_WORDS * (size_t)slot + 8 * sec;
 }
 
 // OWN: through L1, for a sector that this thread itself wrote in this kernel (wf_bounces).
@@ -126,8 +126,11 @@ __device__ __forceinline__ void st_sec(uint32_t* p, const Sec& s) {
                  : "memory");
 }
 
-// sector 0: origin, direction, the trace's start, the depth word
-__device__ __forceinline__ Sec ray_sec(V3 o, V3 d, float start, uint32_t mw) {
+// sector 0: origin, direction, `aux`, the depth word.  Compat: aux is the pixel's minstd state (31 bits), its
+// top bit set while the ray is a re-hit, whose start then waits in sector 1's hit distance.  Clean: aux is
+// the trace's start.
+constexpr uint32_t RAY_REHIT = 0x80000000u;
+__device__ __forceinline__ Sec ray_sec(V3 o, V3 d, uint32_t aux, uint32_t mw) {
     Sec s;
     s.w[0] = __float_as_uint(o.x);
     s.w[1] = __float_as_uint(o.y);
@@ -135,7 +138,7 @@ __device__ __forceinline__ Sec ray_sec(V3 o, V3 d, float start, uint32_t mw) {
     s.w[3] = __float_as_uint(d.x);
     s.w[4] = __float_as_uint(d.y);
     s.w[5] = __float_as_uint(d.z);
-    s.w[6] = __float_as_uint(start);
+    s.w[6] = aux;
     s.w[7] = mw;
     return s;
 }
@@ -144,8 +147,9 @@ __device__ __forceinline__ V3 sec_v3(const Sec& s, int k) {
 }
 __device__ __forceinline__ float sec_f(const Sec& s, int k) { return __uint_as_float(s.w[k]); }
 
-// sector 1: attenuation, sample radiance (the hit words are the extend kernel's to write)
-__device__ __forceinline__ Sec shade_sec(RGB att, RGB acc) {
+// sector 1: attenuation, sample radiance (the hit words are the extend kernel's to write; a compat re-hit
+// leaves its start in the first of them)
+__device__ __forceinline__ Sec shade_sec(RGB att, RGB acc, float start = 0.0f) {
     Sec s;
     s.w[0] = __float_as_uint(att.r);
     s.w[1] = __float_as_uint(att.g);
@@ -153,7 +157,7 @@ __device__ __forceinline__ Sec shade_sec(RGB att, RGB acc) {
     s.w[3] = __float_as_uint(acc.r);
     s.w[4] = __float_as_uint(acc.g);
     s.w[5] = __float_as_uint(acc.b);
-    s.w[6] = 0u;
+    s.w[6] = __float_as_uint(start);
     s.w[7] = 0xffffffffu;
     return s;
 }
@@ -164,7 +168,7 @@ __device__ __forceinline__ void st_hit(uint32_t* shade_sector, float t, uint32_t
                  : "memory");
 }
 
-// sector 2: pixel, sample, minstd state / sample group, PCG32 state, pixel sum
+// sector 2: pixel, sample, sample group, PCG32 state, pixel sum
 __device__ __forceinline__ Sec pixel_sec(uint32_t pixel, uint32_t sample, uint32_t aux, uint64_t pcg_state, float4 ps) {
     Sec s;
     s.w[0] = pixel;
@@ -181,10 +185,18 @@ __device__ __forceinline__ float4 sec_psum(const Sec& s) {
     return make_float4(__uint_as_float(s.w[4]), __uint_as_float(s.w[5]), __uint_as_float(s.w[6]), 0.0f);
 }
 
-// A slot's ray sector carries the start of its trace: 0 for an ordinary ray (tmin = 1e-5,
-// SHADOW_ACNE_FIX, constants.cuh:27), or t + 0.001 for the re-hit from behind a one-sided light that
-// the shade kernel hands back to the extend kernel (camera.cuh:177-183).
-__device__ __forceinline__ float wf_tmin(float start) { return start > 0.0f ? start : 0.00001f; }
+// A trace starts at 1e-5 (SHADOW_ACNE_FIX, constants.cuh:27), or at t + 0.001 for the re-hit from behind a
+// one-sided light that the shade kernel hands back to the extend kernel (camera.cuh:177-183).
+template <bool CLEAN>
+__device__ __forceinline__ bool ray_rehit(const Sec& R) {
+    return CLEAN ? sec_f(R, 6) > 0.0f : (R.w[6] & RAY_REHIT) != 0u;
+}
+// `hit_word`: sector 1's hit distance as the shade step left it (compat; read only for a re-hit).
+template <bool CLEAN, class F>
+__device__ __forceinline__ float ray_tmin(const Sec& R, F hit_word) {
+    if (!ray_rehit<CLEAN>(R)) return 0.00001f;
+    return CLEAN ? sec_f(R, 6) : __uint_as_float(hit_word());
+}
 
 // Work distribution of the iteration kernels, in chunks of 32 queue entries per warp:
 //   fixed    warp w of the grid takes chunks w, w + W, w + 2W, ... (W warps in the grid);
@@ -247,16 +259,23 @@ struct WfRngT<true> {
 template <bool CLEAN>
 using WfRng = typename WfRngT<CLEAN>::type;
 
-// The stream of a slot from its pixel sector: compat keeps the minstd state in word 2; clean keeps the
-// PCG32 state in words 3 and 7, and the increment of sample s's stream is 2 s + 1 (Pcg32::seed).
+// The stream of a slot: compat keeps the minstd state in the ray sector, which every bounce moves anyway;
+// clean keeps the PCG32 state in words 3 and 7 of the pixel sector, and the increment of sample s's stream
+// is 2 s + 1 (Pcg32::seed).
 template <bool CLEAN>
-__device__ __forceinline__ void rng_load(const Sec& px, WfRng<CLEAN>& r) {
+__device__ __forceinline__ void rng_load(const Sec& R, const Sec& px, WfRng<CLEAN>& r) {
     if constexpr (CLEAN) {
         r.state = ((uint64_t)px.w[7] << 32) | px.w[3];
         r.inc = ((uint64_t)px.w[1] << 1) | 1u;
     } else {
-        r.x = px.w[2];
+        r.x = R.w[6] & ~RAY_REHIT;
     }
+}
+// The ray sector's aux word of an ordinary ray.
+template <bool CLEAN>
+__device__ __forceinline__ uint32_t ray_aux(const WfRng<CLEAN>& r) {
+    if constexpr (CLEAN) return 0u;
+    else return r.x;
 }
 
 
@@ -285,14 +304,12 @@ __device__ __forceinline__ void wf_start_sample(const DevScene& S, const DevPara
     }
 }
 
-// The pixel sector's stream words after `rng` has advanced (compat: word 2; clean: words 3 and 7).
+// The pixel sector's stream words after `rng` has advanced (clean: words 3 and 7; compat has none).
 template <bool CLEAN>
 __device__ __forceinline__ void rng_store(Sec& px, const WfRng<CLEAN>& rng) {
     if constexpr (CLEAN) {
         px.w[3] = (uint32_t)rng.state;
         px.w[7] = (uint32_t)(rng.state >> 32);
-    } else {
-        px.w[2] = rng.x;
     }
 }
 
@@ -394,9 +411,9 @@ __device__ __forceinline__ bool wf_fetch_pixel(const J& jobs, const WfWindow& wi
     if constexpr (!CLEAN) rng.seed(P.seed + pixel);
     Ray r;
     wf_start_sample<CLEAN, ORDER>(S, P, rng, pixel, s0, r);
-    st_sec(wf_sec(B, slot, SEC_RAY), ray_sec(r.o, r.d, 0.0f, wf_pack((uint32_t)P.max_depth, job)));
+    st_sec(wf_sec(B, slot, SEC_RAY), ray_sec(r.o, r.d, ray_aux<CLEAN>(rng), wf_pack((uint32_t)P.max_depth, job)));
     st_sec(wf_sec(B, slot, SEC_SHADE), shade_sec(rgb(1.f, 1.f, 1.f), rgb(0.f, 0.f, 0.f)));
-    Sec px = pixel_sec(pixel, s0, grp, 0ull, make_float4(0.f, 0.f, 0.f, 0.f));   // clean: word 2 = group
+    Sec px = pixel_sec(pixel, s0, grp, 0ull, make_float4(0.f, 0.f, 0.f, 0.f));
     rng_store<CLEAN>(px, rng);
     st_sec(wf_sec(B, slot, SEC_PIXEL), px);
     return true;
@@ -496,11 +513,13 @@ __global__ void RTC_EXTEND_BOUNDS wf_extend(J jobs, WfBuffers B, WfIter w, unsig
             float t;
             uint32_t item;
             constexpr int WALK = !WIDE ? WALK_BINARY : std::is_same<J, WfOne>::value ? WALK_WIDE : WALK_EITHER;
-            bool h = closest_hit<FLAVOR == 2, WALK>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), wf_tmin(sec_f(R, 6)),
+            uint32_t* sh = wf_sec(B, slot, SEC_SHADE);
+            const float tmin = ray_tmin<FLAVOR == 2>(R, [&] { return ld_word(sh + 6); });
+            bool h = closest_hit<FLAVOR == 2, WALK>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), tmin,
                                                     3.402823466e+38f,
                                                     wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t, item, st,
                                                     status);
-            st_hit(wf_sec(B, slot, SEC_SHADE), t, h ? item : 0xffffffffu);
+            st_hit(sh, t, h ? item : 0xffffffffu);
             ++rays;
         }
         chunks.advance(pending);   // one call site: every lane of the warp takes part
@@ -542,10 +561,10 @@ __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, cons
     r.time = 0.0f;
     RGB att = rgb(sec_f(SH, 0), sec_f(SH, 1), sec_f(SH, 2)), acc = rgb(sec_f(SH, 3), sec_f(SH, 4), sec_f(SH, 5));
     WfRng<CLEAN> rng;
-    rng_load<CLEAN>(PX, rng);   // of the pixel sector only the stream is kept past this point
+    rng_load<CLEAN>(R, PX, rng);   // of the pixel sector only clean mode's stream is read before the sample ends
     uint32_t depth = wf_depth(R.w[7]);
     float rehit_tmin = 0.0f;
-    const int out = shade_bounce_deferred<CLEAN, ORDER>(S, r, item != 0xffffffffu, t, item, sec_f(R, 6) > 0.0f, acc,
+    const int out = shade_bounce_deferred<CLEAN, ORDER>(S, r, item != 0xffffffffu, t, item, ray_rehit<CLEAN>(R), acc,
                                                         att, rng, status, rehit_tmin);
     uint32_t* rec_ray = wf_sec(B, slot, SEC_RAY);
     uint32_t* rec_shade = wf_sec(B, slot, SEC_SHADE);
@@ -553,21 +572,20 @@ __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, cons
     if (out == BOUNCE_REHIT) {
         // the same ray again from behind the light, at the same depth: only the radiance and the ray's
         // start change (no random draw has been made)
-        st_sec(rec_ray, ray_sec(r.o, r.d, rehit_tmin, R.w[7]));
-        st_sec(rec_shade, shade_sec(att, acc));
+        const uint32_t aux = CLEAN ? __float_as_uint(rehit_tmin) : ray_aux<CLEAN>(rng) | RAY_REHIT;
+        st_sec(rec_ray, ray_sec(r.o, r.d, aux, R.w[7]));
+        st_sec(rec_shade, shade_sec(att, acc, CLEAN ? 0.0f : rehit_tmin));
         return true;
     }
     const bool cont = out == BOUNCE_NEXT;
     if (cont) --depth;
     if (cont && depth > 0u) {
-        // the path continues: next bounce (of the pixel sector only the stream words change)
-        st_sec(rec_ray, ray_sec(r.o, r.d, 0.0f, wf_pack(depth, job)));
+        // the path continues: next bounce (of the pixel sector only clean mode's stream words change)
+        st_sec(rec_ray, ray_sec(r.o, r.d, ray_aux<CLEAN>(rng), wf_pack(depth, job)));
         st_sec(rec_shade, shade_sec(att, acc));
         if constexpr (CLEAN) {
             st_word(rec_px + 3, (uint32_t)rng.state);
             st_word(rec_px + 7, (uint32_t)(rng.state >> 32));
-        } else {
-            st_word(rec_px + 2, rng.x);
         }
         return true;
     }
@@ -588,7 +606,7 @@ __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, cons
         // regenerate: the pixel's next sample on the same slot
         Ray nr;
         wf_start_sample<CLEAN, ORDER>(S, P, rng, pixel, s, nr);
-        st_sec(rec_ray, ray_sec(nr.o, nr.d, 0.0f, wf_pack((uint32_t)P.max_depth, job)));
+        st_sec(rec_ray, ray_sec(nr.o, nr.d, ray_aux<CLEAN>(rng), wf_pack((uint32_t)P.max_depth, job)));
         st_sec(rec_shade, shade_sec(rgb(1.f, 1.f, 1.f), rgb(0.f, 0.f, 0.f)));
         Sec npx = pixel_sec(pixel, s, px.w[2], 0ull, ps);
         rng_store<CLEAN>(npx, rng);
@@ -642,7 +660,8 @@ __device__ __forceinline__ void wf_shade_pass(const J& jobs, const WfBuffers& B,
             slot = ld_state(q + k);
             const Sec R = ld_sec(wf_sec(B, slot, SEC_RAY));
             const Sec SH = ld_sec(wf_sec(B, slot, SEC_SHADE));
-            const Sec PX = ld_sec(wf_sec(B, slot, SEC_PIXEL));
+            Sec PX{};
+            if constexpr (CLEAN) PX = ld_sec(wf_sec(B, slot, SEC_PIXEL));
             live = wf_step<CLEAN, ORDER>(jobs, win, B, slot, R, SH, PX, sec_f(SH, 6), SH.w[7], pc, st, paths, status);
         }
         wf_push(qn, cn, slot, live);
@@ -706,14 +725,15 @@ __global__ void __launch_bounds__(WF_BOUNCES_BLOCK, 20) wf_bounces(J jobs, WfBuf
             if (live) {
                 const Sec R = ld_sec<true>(wf_sec(B, slot, SEC_RAY));
                 const Sec SH = ld_sec<true>(wf_sec(B, slot, SEC_SHADE));
-                const Sec PX = ld_sec<true>(wf_sec(B, slot, SEC_PIXEL));
+                Sec PX{};
+                if constexpr (CLEAN) PX = ld_sec<true>(wf_sec(B, slot, SEC_PIXEL));
                 const uint32_t mw = R.w[7];
                 const uint32_t job = wf_job(mw);
                 float t;
                 uint32_t item;
-                const bool h = closest_hit<CLEAN>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), wf_tmin(sec_f(R, 6)),
-                                                  3.402823466e+38f, wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t,
-                                                  item, st, status);
+                const bool h = closest_hit<CLEAN>(jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3),
+                                                  ray_tmin<CLEAN>(R, [&] { return SH.w[6]; }), 3.402823466e+38f,
+                                                  wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t, item, st, status);
                 live = wf_step<CLEAN, ORDER, true>(jobs, win, B, slot, R, SH, PX, t, h ? item : 0xffffffffu, pc, st, paths,
                                                    status);
             }
@@ -776,14 +796,14 @@ __device__ __forceinline__ void drain_load(const WfBuffers& B, uint32_t slot, Dr
               PX = ld_sec(wf_sec(B, slot, SEC_PIXEL));
     x.o = sec_v3(R, 0);
     x.d = sec_v3(R, 3);
-    x.tmin = wf_tmin(sec_f(R, 6));
+    x.tmin = ray_tmin<CLEAN>(R, [&] { return SH.w[6]; });
     x.mw = R.w[7];
     x.att = rgb(sec_f(SH, 0), sec_f(SH, 1), sec_f(SH, 2));
     x.acc = rgb(sec_f(SH, 3), sec_f(SH, 4), sec_f(SH, 5));
     x.pr = sec_f(PX, 4);
     x.pg = sec_f(PX, 5);
     x.pb = sec_f(PX, 6);
-    rng_load<CLEAN>(PX, x.rng);
+    rng_load<CLEAN>(R, PX, x.rng);
     x.pixel = PX.w[0];
     x.sample = PX.w[1];
     x.grp = CLEAN ? PX.w[2] : 0u;
