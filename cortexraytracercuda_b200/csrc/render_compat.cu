@@ -96,12 +96,13 @@ __global__ void __launch_bounds__(128) rtc_trace_closest(DevScene S, const float
                                                          uint32_t* status_word) {
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const float* R = rays + 8 * (size_t)k;
-    V3 o = v3(R[0], R[1], R[2]), d = v3(R[4], R[5], R[6]);
+    const float4* R = (const float4*)rays + 2 * (size_t)k;   // (origin, tmin) (direction, tmax): two 16-byte loads
+    const float4 r0 = __ldg(R), r1 = __ldg(R + 1);
+    V3 o = v3(r0.x, r0.y, r0.z), d = v3(r1.x, r1.y, r1.z);
     float t;
     uint32_t item, status = 0;
     TraceStats st{0, 0};
-    bool h = closest_hit<false, WIDE ? WALK_WIDE : WALK_BINARY>(S, o, d, R[3], R[7], depth == max_depth, t, item, st, status);
+    bool h = closest_hit<false, WIDE ? WALK_WIDE : WALK_BINARY>(S, o, d, r0.w, r1.w, depth == max_depth, t, item, st, status);
     if (prim) prim[k] = h ? item_gid(S, item) : -1;
     if (tout) tout[k] = h ? t : INFINITY;
     if (status) atomicOr(status_word, status);

@@ -92,6 +92,7 @@ extern "C" rtc_status rtc_context_destroy(rtc_context* c) {
     cudaFree(c->d_wf);
     cudaFree(c->d_groups);
     cudaFree(c->d_batch_groups);
+    cudaFree(c->d_trace);
     if (c->h_poll) cudaFreeHost(c->h_poll);
     for (cudaEvent_t& e : c->poll_ev)
         if (e) cudaEventDestroy(e);
@@ -1496,6 +1497,9 @@ extern "C" rtc_status rtc_get_render_stats(rtc_context* c, rtc_render_stats* out
     return RTC_OK;
 }
 
+// Ray and hit buffers up to this size (1.6 M rays) stay with the context; larger calls return theirs.
+constexpr size_t TRACE_KEEP_BYTES = size_t(64) << 20;
+
 extern "C" rtc_status rtc_trace_closest(rtc_context* c, const rtc_scene* s, const float* rays, uint32_t n,
                                         int32_t depth, int32_t max_depth, int32_t* prim, float* t) {
     return rtc_trace_closest_ex(c, s, rays, n, depth, max_depth, 0, prim, t);
@@ -1508,31 +1512,39 @@ extern "C" rtc_status rtc_trace_closest_ex(rtc_context* c, const rtc_scene* s, c
     std::lock_guard<std::mutex> lk(c->mu);
     RtcDeviceScope dev(c->device);
     RTC_CUDA(dev.error());
-    float* d_rays = nullptr;
-    int32_t* d_prim = nullptr;
-    float* d_t = nullptr;
-    cudaError_t e = cudaMalloc(&d_rays, (size_t)n * 8 * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&d_prim, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&d_t, (size_t)n * 4);
-    rtc_status r = RTC_OK;
-    if (e != cudaSuccess) r = cuda_fail(e, "cudaMalloc(trace)");
-    if (r == RTC_OK) {
-        e = cudaMemcpyAsync(d_rays, rays, (size_t)n * 8 * sizeof(float), cudaMemcpyHostToDevice, c->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, 4, c->stream);
-        rtc_render_params vp{};
-        vp.flags = flags;
-        const DevScene SV = rtc_scene_view(s, &vp);
-        auto tfn = SV.num_xnodes ? rtc_launch_trace_closest_x : rtc_launch_trace_closest;
-        if (e == cudaSuccess) e = tfn(SV, d_rays, n, depth, max_depth, d_prim, d_t, c->d_status, c->stream);
-        if (e == cudaSuccess && prim) e = cudaMemcpyAsync(prim, d_prim, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess && t) e = cudaMemcpyAsync(t, d_t, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-        if (e != cudaSuccess) r = cuda_fail(e, "trace_closest");
+    // rays (32 bytes each), ids and distances in one block, kept with the context while it is small: three
+    // allocations and three frees a call cost more than the trace itself (200,003 rays against 61 K
+    // triangles: 1.95 -> 0.64 ms)
+    const size_t rays_bytes = (size_t)n * 8 * sizeof(float), bytes = rays_bytes + (size_t)n * 8;
+    void* block = nullptr;
+    if (bytes <= TRACE_KEEP_BYTES) {
+        if (c->trace_cap < bytes) {
+            cudaFree(c->d_trace);
+            c->d_trace = nullptr;
+            c->trace_cap = 0;
+            RTC_CUDA(cudaMalloc(&c->d_trace, bytes));
+            c->trace_cap = bytes;
+        }
+        block = c->d_trace;
+    } else {
+        RTC_CUDA(cudaMalloc(&block, bytes));
     }
-    cudaFree(d_rays);
-    cudaFree(d_prim);
-    cudaFree(d_t);
-    if (r != RTC_OK) return r;
+    float* d_rays = (float*)block;
+    int32_t* d_prim = (int32_t*)((uint8_t*)block + rays_bytes);
+    float* d_t = (float*)(d_prim + n);
+    cudaError_t e = cudaMemcpyAsync(d_rays, rays, rays_bytes, cudaMemcpyHostToDevice, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, 4, c->stream);
+    rtc_render_params vp{};
+    vp.flags = flags;
+    const DevScene SV = rtc_scene_view(s, &vp);
+    auto tfn = SV.num_xnodes ? rtc_launch_trace_closest_x : rtc_launch_trace_closest;
+    if (e == cudaSuccess) e = tfn(SV, d_rays, n, depth, max_depth, d_prim, d_t, c->d_status, c->stream);
+    if (e == cudaSuccess && prim) e = cudaMemcpyAsync(prim, d_prim, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
+    if (e == cudaSuccess && t) e = cudaMemcpyAsync(t, d_t, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
+    const cudaError_t e2 = cudaStreamSynchronize(c->stream);   // also before the block is freed or reused
+    if (e == cudaSuccess) e = e2;
+    if (block != c->d_trace) cudaFree(block);
+    if (e != cudaSuccess) return cuda_fail(e, "trace_closest");
     return read_status(c);
 }
 

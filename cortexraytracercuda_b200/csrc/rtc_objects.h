@@ -30,6 +30,8 @@ struct rtc_context {
     size_t groups_cap = 0;
     void* d_batch_groups = nullptr;    // the same for the images of a batch
     size_t batch_groups_cap = 0;
+    void* d_trace = nullptr;           // rtc_trace_closest: rays and hits (kept up to TRACE_KEEP_BYTES)
+    size_t trace_cap = 0;
     uint32_t* h_poll = nullptr;       // pinned: queue sizes read back between batches
     cudaEvent_t poll_ev[2] = {nullptr, nullptr};
     cudaEvent_t phase_ev[3] = {nullptr, nullptr, nullptr};   // render start, drain start, render end

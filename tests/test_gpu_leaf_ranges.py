@@ -84,3 +84,18 @@ def test_transformed_runs(ctx, n, transforms):
     ds = DeviceScene(ctx, scene)
     _check(ds, want, rays)
     _check(ds, want, rays, FLAG_WIDE_BVH)
+
+
+def test_trace_block_sizes(ctx):
+    """Ray queries of growing and shrinking size share the context's kept block; the last is past what is
+    kept (1,677,721 rays) and uses its own.  Every call gives each ray the hit that it has in a call alone."""
+    scene = _scene(("sphere", "tri", "quad"), 40, 5)
+    ds = DeviceScene(ctx, scene)
+    rays = _rays(1000, 3)
+    prim, t = ds.trace_closest(rays, 0, 8)
+    oracle_prim, oracle_t = oracles.port().scene(scene).trace_closest(rays, 0, 8)
+    assert np.array_equal(prim, oracle_prim) and np.array_equal(t[prim >= 0], oracle_t[prim >= 0])
+    for n in (1, 33, 5000, 127, 200_003, 1_677_722, 64):
+        reps = -(-n // 1000)
+        p, tt = ds.trace_closest(np.tile(rays, (reps, 1))[:n], 0, 8)
+        assert np.array_equal(p, np.tile(prim, reps)[:n]) and np.array_equal(tt, np.tile(t, reps)[:n])
