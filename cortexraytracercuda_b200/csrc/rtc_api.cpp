@@ -1169,12 +1169,14 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     // make a bounce instruction-bound, where packing pays (5-15% of a frame at 16 or more spp); elsewhere
     // the longest chains' latency bounds the drain and repacking costs 2-50% (wf_finish, wf_finish_packed).
     L.drain_every = rtc_drain_every(S.num_xnodes ? 2 : 0);
-    // Work distribution of the iteration kernels.  Extend: one 32-entry chunk per warp, the grid as long as
-    // the queue can be, so that the block scheduler balances uneven walks and no launch ends on the stride's
-    // last, half-empty round (8 blocks per SM striding the queue: spheres frame 54.7 against 53.7 ms, a
-    // 20,480-triangle frame with the 8-wide nodes 15.2 against 14.4).  From 2^20 primitives on, chunks handed out by a counter to
+    // Work distribution of the iteration kernels.  Extend: a grid as long as the queue can be, up to four
+    // resident waves (32 blocks per SM), so that the block scheduler balances uneven walks and a launch does
+    // not end on a half-empty round of one wave's stride (one wave: spheres frame 54.7 against 53.7 ms, an
+    // 81,920-triangle frame with the 8-wide nodes 15.2 against 14.4); a longer grid gains nothing more and
+    // costs where the queue has run empty before the host knows (3.3 M pixels of one sample: 1.28 ms with
+    // the whole queue's grid, 1.07 with this).  From 2^20 primitives on, chunks handed out by a counter to
     // 8 blocks per SM, whose warps keep their place in the caches (1.31 M triangles: extend 49.8 ms against
-    // 50.2 with the long grid and 53.8 with the stride).  Shade: 8 blocks per SM striding the queue (one
+    // 50.2 with the long grid and 53.8 with one wave's stride).  Shade: 8 blocks per SM striding the queue (one
     // resident wave; the long grid costs it 5-15%); the counter costs it more than it balances (same frame: 10.1
     // against 8.3 ms), but clean mode keeps it in those scenes, where the two kernels round a refraction
     // differently in the last bit.
@@ -1264,7 +1266,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
             it += BATCH;
             ++run.launches;
         } else {
-            const int long_grid = (int)std::max<int64_t>(1, (bound + 127) / 128);   // 128-thread blocks
+            const int long_grid = (int)std::min<int64_t>(std::max<int64_t>(1, (bound + 127) / 128), (int64_t)grid * 4);
             for (int k = 0; k < BATCH; ++k, ++it) {
                 L.w = wf_iter(rot++);
                 L.dynamic = dynamic_extend;
