@@ -14,6 +14,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
@@ -100,6 +101,12 @@ private:
     rtc_status observe(int slot);
     rtc_status enqueue_iterations();
     void drop_graph();
+    // Whether every unit not yet claimed has an idle slot waiting for it, by what was last observed (late, so
+    // on the safe side): from here on the queue only runs down.
+    bool runs_down() const {
+        const uint64_t unclaimed = limit_ - std::min(next_, limit_);
+        return unclaimed + live_ <= cfg_.slots;
+    }
 
     EngineConfig cfg_;
     cudaStream_t st_ = nullptr;
@@ -134,8 +141,9 @@ private:
     std::vector<uint64_t> completed_;
     uint64_t it_ = 0, launches_ = 0;
     // six (extend, shade) iterations captured once: the queue rotation repeats every six iterations,
-    // so the same graph serves every batch that starts at a multiple of six
-    cudaGraphExec_t graph_ = nullptr;
+    // so the same graph serves every batch that starts at a multiple of six; one graph for a queue that is
+    // kept full, one for a queue that runs down (enqueue_iterations)
+    cudaGraphExec_t graph_[2] = {nullptr, nullptr};
     unsigned long long* graph_counters_ = nullptr;
 };
 
