@@ -1260,7 +1260,9 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
         if (bounces) {
             L.w = wf_iter(rot++);
             L.steps = BATCH;
-            L.grid = (int)std::max<int64_t>(1, (bound + rtc::WF_BOUNCES_BLOCK - 1) / rtc::WF_BOUNCES_BLOCK);
+            const int64_t warps = (int64_t)num_sms * 8;   // a shorter queue is spread over this many
+            L.per = (uint32_t)std::min<int64_t>(rtc::WF_BOUNCES_BLOCK, std::max<int64_t>(1, (bound + warps - 1) / warps));
+            L.grid = (int)std::max<int64_t>(1, (bound + L.per - 1) / L.per);
             e = fn(WF_OP_BOUNCES, J, B, L);
             if (e != cudaSuccess) return cuda_fail(e, "wavefront iterations");
             it += BATCH;

@@ -37,6 +37,7 @@ struct WfLaunch {
     WfIter w;
     WfWindow win;                    // ADMIT: the window to publish
     int steps;                       // BOUNCES: bounces per slot
+    uint32_t per;                    // BOUNCES: queue entries a block takes at a time (1 to its 32 lanes)
     float k0, threshold;             // SPLIT: iterations so far, long-chain threshold (iterations)
     bool wide;                       // EXTEND: walk the 8-wide nodes (where the scene carries them)
     unsigned long long* counters;    // NULL: no instrumentation

@@ -704,9 +704,11 @@ __global__ void RTC_SHADE_BOUNDS wf_shade_ring(WfTable jobs, WfBuffers B, WfIter
 // 4,096 slots per SM against the split kernels only: spheres 1280x720 55.5 / 54.9 / 55.2 against 56.8 ms,
 // meshes (1.31 M triangles) 62.9 / 62.3 / 62.3 against 64.1, transforms 333x251 7.00 / 6.90 / 6.91 against
 // 7.24; Cornell 256x256 1.60 against 1.79, 64x48 preview 0.26 against 0.44 ms.  96 registers (20 warps per
-// SM) beat 128: spheres 54.9 against 55.9 ms.
+// SM) beat 128: spheres 54.9 against 55.9 ms.  A block takes `per` entries at a time: all 32 of its lanes',
+// or fewer for a queue so short that full warps would leave SMs idle (rule in run_wavefront: at most 8 warps
+// per SM; 64x48 preview 0.236 -> 0.190 ms, nothing to gain from 65,536 slots on).
 template <bool CLEAN, int ORDER, class J>
-__global__ void __launch_bounds__(WF_BOUNCES_BLOCK, 20) wf_bounces(J jobs, WfBuffers B, WfIter w, int steps,
+__global__ void __launch_bounds__(WF_BOUNCES_BLOCK, 20) wf_bounces(J jobs, WfBuffers B, WfIter w, int steps, uint32_t per,
                                                                    uint32_t* status_word) {
     const uint32_t n = B.ctr[w.cin];
     if (blockIdx.x == 0 && threadIdx.x == 0) B.ctr[w.czero] = 0u;   // appended to by the next iteration
@@ -715,10 +717,11 @@ __global__ void __launch_bounds__(WF_BOUNCES_BLOCK, 20) wf_bounces(J jobs, WfBuf
     uint32_t status = 0, paths = 0;
     PathCounters pc{0, 0, 0};
     TraceStats st{0, 0};
-    const uint32_t stride = gridDim.x * WF_BOUNCES_BLOCK;
-    for (uint32_t base = blockIdx.x * WF_BOUNCES_BLOCK; base < n; base += stride) {   // whole warps
+    // spread over the warps there are
+    if (per < WF_BOUNCES_BLOCK) per = min((uint32_t)WF_BOUNCES_BLOCK, (n + gridDim.x - 1u) / gridDim.x);
+    for (uint32_t base = blockIdx.x * per; base < n; base += gridDim.x * per) {   // the same for the whole warp
         const uint32_t k = base + threadIdx.x;
-        bool live = k < n;
+        bool live = threadIdx.x < per && k < n;
         uint32_t slot = 0;
         if (live) slot = ld_state(q + k);
         for (int s = 0; s < steps && __any_sync(0xffffffffu, live); ++s) {
@@ -1070,7 +1073,7 @@ cudaError_t wf_dispatch(WfOp op, const A& args, const WfBuffers& B, const WfLaun
     case WF_OP_BOUNCES:
         // one image only: a ring's slots take new pixels at every iteration
         if constexpr (std::is_same<J, WfOne>::value)
-            wf_bounces<CLEAN, ORDER><<<L.grid, WF_BOUNCES_BLOCK, 0, L.st>>>(jobs, B, L.w, L.steps, L.status);
+            wf_bounces<CLEAN, ORDER><<<L.grid, WF_BOUNCES_BLOCK, 0, L.st>>>(jobs, B, L.w, L.steps, L.per, L.status);
         else return cudaErrorInvalidValue;
         break;
     default:
