@@ -442,13 +442,15 @@ rtc_status rtc_render(rtc_context* ctx, const rtc_scene* scene, const rtc_render
  * and receives: rays traced (closest-hit traversals), paths traced, BVH nodes visited, primitive
  * tests, then the wavefront extend kernel's own rays, node visits and primitive tests, one unused.  The megakernel engine
  * returns without waiting for the GPU; the wavefront engine polls its queue counter between batches
- * of iterations and returns once the frame is complete. */
+ * of iterations (a frame of fewer than 512 work units per SM is queued without a poll).  The last
+ * kernels may still run when it returns, in order on `stream`.  A stream under capture is refused. */
 rtc_status rtc_render_device(rtc_context* ctx, const rtc_scene* scene, const rtc_render_params* params,
                              float* d_radiance_sum, uint8_t* d_rgb8, unsigned long long* d_counters,
                              void* stream);
 
 /* Statistics of the last render on this context (wavefront engine): iterations of (extend, shade),
- * kernel launches, whether the drain kernel ran and for how many slots, and the device time of the
+ * kernel launches, whether the drain kernel ran and for how many slots (at most, where the frame was
+ * queued without a poll), and the device time of the
  * bulk iterations and of the drain kernel (ms, from CUDA events; the call waits for the render). */
 typedef struct rtc_render_stats {
     uint32_t iterations;
