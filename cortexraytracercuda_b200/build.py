@@ -47,6 +47,15 @@ SOURCES = [
     ("wavefront_compat.cu", "wavefront_compat_dev_x", "nvcc", ["--fmad=true", "-DRTC_FLAVOR=0", "-DRTC_XP=1"]),
     ("render_clean.cu", "render_clean_x", "nvcc", ["--fmad=true", "-DRTC_XP=1"]),
     ("wavefront_clean.cu", "wavefront_clean_x", "nvcc", ["--fmad=true", "-DRTC_XP=1"]),
+    # the one-image wavefront kernels without the code that plain scenes do not reach (RTC_PLAIN=1)
+    ("wavefront_compat.cu", "wavefront_compat_host_p", "nvcc", ["--fmad=false", "-DRTC_FLAVOR=1", "-DRTC_PLAIN=1"]),
+    ("wavefront_compat.cu", "wavefront_compat_dev_p", "nvcc", ["--fmad=true", "-DRTC_FLAVOR=0", "-DRTC_PLAIN=1"]),
+    ("wavefront_clean.cu", "wavefront_clean_p", "nvcc", ["--fmad=true", "-DRTC_PLAIN=1"]),
+    ("wavefront_compat.cu", "wavefront_compat_host_xp", "nvcc",
+     ["--fmad=false", "-DRTC_FLAVOR=1", "-DRTC_XP=1", "-DRTC_PLAIN=1"]),
+    ("wavefront_compat.cu", "wavefront_compat_dev_xp", "nvcc",
+     ["--fmad=true", "-DRTC_FLAVOR=0", "-DRTC_XP=1", "-DRTC_PLAIN=1"]),
+    ("wavefront_clean.cu", "wavefront_clean_xp", "nvcc", ["--fmad=true", "-DRTC_XP=1", "-DRTC_PLAIN=1"]),
     ("render_noalloc.cu", "render_noalloc", "nvcc", []),
     ("rtc_api.cpp", "rtc_api", "cxx", []),
     ("rtc_engine.cpp", "rtc_engine", "cxx", []),

@@ -862,6 +862,10 @@ rtc_status rtc_build_host_scene(const rtc_scene_desc* d, HostScene& H, uint32_t 
     D.bg.env_w = d->background.env_width;
     D.bg.env_h = d->background.env_height;
     D.bg.cdf = env_cdf.empty() ? nullptr : (const float*)off(o_envcdf);
+    bool sphere_light = false;
+    for (uint32_t i = 0; i < nlights; ++i) sphere_light = sphere_light || light[6 * (size_t)i + 4].w < 0.0f;
+    D.plain = !D.num_images && (D.bg.kind == 0 || D.bg.kind == 1) && !D.bg.cdf && tri_vn.empty() && tri_uv.empty() &&
+              !sphere_light;
     D.bg.pdf_scale = env_cdf.empty() ? 0.0f
                                      : (float)((double)D.bg.env_w * D.bg.env_h /
                                                (2.0 * 3.14159265358979323846 * 3.14159265358979323846));
@@ -1115,10 +1119,13 @@ struct WfTimer {
 };
 
 // `xp`: the scene has transformed primitives or boxes (an xprim BVH), walked by the RTC_XP=1 kernels.
-rtc::WfOneFn wf_one_fn(const rtc_render_params* p, bool xp) {
-    if (p->mode == RTC_MODE_CLEAN) return xp ? rtc_wf_one_clean_x : rtc_wf_one_clean;
-    if (p->draw_order == RTC_DRAW_ORDER_HOST) return xp ? rtc_wf_one_compat_host_x : rtc_wf_one_compat_host;
-    return xp ? rtc_wf_one_compat_dev_x : rtc_wf_one_compat_dev;
+rtc::WfOneFn wf_one_fn(const rtc_render_params* p, const rtc::DevScene& S) {
+    static const rtc::WfOneFn fn[3][2][2] = {   // [clean, g++ flavour, nvcc flavour][xprims][plain]
+        {{rtc_wf_one_clean, rtc_wf_one_clean_p}, {rtc_wf_one_clean_x, rtc_wf_one_clean_xp}},
+        {{rtc_wf_one_compat_host, rtc_wf_one_compat_host_p}, {rtc_wf_one_compat_host_x, rtc_wf_one_compat_host_xp}},
+        {{rtc_wf_one_compat_dev, rtc_wf_one_compat_dev_p}, {rtc_wf_one_compat_dev_x, rtc_wf_one_compat_dev_xp}}};
+    const int m = p->mode == RTC_MODE_CLEAN ? 0 : p->draw_order == RTC_DRAW_ORDER_HOST ? 1 : 2;
+    return fn[m][S.num_xnodes != 0][S.plain != 0];
 }
 
 rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const WfBuffers& B, uint32_t* d_status,
@@ -1133,7 +1140,7 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     DevParams P = dev_params(p);
     P.rgb8 = d_rgb8;   // quantised output written as each pixel finishes
     const bool clean = p->mode == RTC_MODE_CLEAN;
-    const WfOneFn fn = wf_one_fn(p, S.num_xnodes != 0);
+    const WfOneFn fn = wf_one_fn(p, S);
     WfOneArgs J;
     J.S = S;
     J.P = P;

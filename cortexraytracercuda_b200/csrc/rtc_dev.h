@@ -57,13 +57,30 @@
 #ifndef RTC_XP
 #define RTC_XP 0
 #endif
-#if RTC_XP
+// RTC_PLAIN=1 builds the one-image kernels once more for scenes with `DevScene::plain` set, without the code
+// that only other scenes reach: image textures and the texture coordinates that only they read, smooth normals,
+// the environment map, and omni / spot lights.  None of it runs in a plain scene, but it is a good part of the
+// instructions that a bounce's kernels span (their stalls on instruction fetch) and holds registers across them.
+// B200, the full kernels -> these: spheres 1280x720x64 53.2 -> 49.4 ms, Cornell 256x256x16 1.57 -> 1.46, clean
+// spheres 960x540x16 4.34 -> 4.11, transformed primitives 333x251x32 6.9 -> 5.96; the same bits.  Moving that
+// code behind calls instead slowed the drain by 13%.  The job ring, whose scenes mix, keeps the full kernels.
+#ifndef RTC_PLAIN
+#define RTC_PLAIN 0
+#endif
+#if RTC_XP && RTC_PLAIN
+#define RTC_XP_NS xp1p
+#elif RTC_XP
 #define RTC_XP_NS xp1
+#elif RTC_PLAIN
+#define RTC_XP_NS xp0p
 #else
 #define RTC_XP_NS xp0
 #endif
 
 namespace rtc {
+inline namespace RTC_XP_NS {
+constexpr bool PLAIN = RTC_PLAIN != 0;
+}
 
 enum ItemKind : uint32_t { ITEM_SPHERE = 0, ITEM_QUAD = 1, ITEM_TRI = 2, ITEM_LIGHT = 3, ITEM_XPRIM = 4 };
 // Item word: (kind << ITEM_KIND_SHIFT) | index into that kind's array.
@@ -144,6 +161,7 @@ struct DevScene {
     uint32_t num_images;
     uint32_t num_sph, num_tri, num_quad;
     uint32_t num_xprim, num_xf, num_rect, num_xnodes;
+    uint32_t plain;            // nonzero: no image texture, environment map, smooth normal or omni / spot light
     DevCamera cam;
     DevBackground bg;
 };

@@ -12,8 +12,12 @@
 
 #define RTC_FLAVOR_CAT2(a, b) a##b
 #define RTC_FLAVOR_CAT(a, b) RTC_FLAVOR_CAT2(a, b)
-#if RTC_XP
+#if RTC_XP && RTC_PLAIN
+#define RTC_XP_FN(name) RTC_FLAVOR_CAT(name, _xp)
+#elif RTC_XP
 #define RTC_XP_FN(name) RTC_FLAVOR_CAT(name, _x)
+#elif RTC_PLAIN
+#define RTC_XP_FN(name) RTC_FLAVOR_CAT(name, _p)
 #else
 #define RTC_XP_FN(name) name
 #endif
@@ -83,3 +87,12 @@ RTC_DECLARE_COMPAT(_host_x)
                                         const rtc::WfLaunch& L);
 RTC_DECLARE_CLEAN()
 RTC_DECLARE_CLEAN(_x)
+// `_p`, `_xp`: the one-image wavefront kernels built with RTC_PLAIN=1, for scenes with DevScene::plain
+#define RTC_DECLARE_ONE(name) \
+    cudaError_t name(rtc::WfOp op, const rtc::WfOneArgs& a, const rtc::WfBuffers& B, const rtc::WfLaunch& L);
+RTC_DECLARE_ONE(rtc_wf_one_compat_dev_p)
+RTC_DECLARE_ONE(rtc_wf_one_compat_dev_xp)
+RTC_DECLARE_ONE(rtc_wf_one_compat_host_p)
+RTC_DECLARE_ONE(rtc_wf_one_compat_host_xp)
+RTC_DECLARE_ONE(rtc_wf_one_clean_p)
+RTC_DECLARE_ONE(rtc_wf_one_clean_xp)

@@ -119,7 +119,7 @@ __device__ __forceinline__ V3 random_to_sphere(R& rng, float radius, float dista
 template <int ORDER, class R>
 __device__ __forceinline__ V3 light_random(const DevScene& S, uint32_t li, V3 o, R& rng) {
     const float4* q = S.light + 6 * (size_t)li;
-    if (__ldg(q + 4).w < 0.0f) {
+    if (!PLAIN && __ldg(q + 4).w < 0.0f) {
         const float4 c = __ldg(q);
         const V3 dir = sub(v3(c.x, c.y, c.z), o);
         const Onb b = build_from_w(dir);
@@ -234,7 +234,7 @@ __device__ __forceinline__ void scatter_bounce(const DevScene& S, Ray& r, Hit& h
     Onb b = build_from_w(h.n);
     V3 dir;
     float pdf_val, spdf;
-    if (CLEAN && S.bg.cdf) {
+    if (CLEAN && !PLAIN && S.bg.cdf) {
         // with environment-map sampling: mixture_pdf(objects, background, 0.8) (camera.cuh:333-336),
         // objects = the light/cosine mixture below (cosine alone without lights)
         const bool lights = S.num_lights > 0;
@@ -301,7 +301,7 @@ __device__ __forceinline__ RGB emitted(const DevScene& S, const Ray& r, Hit& h, 
             RGB tv = texture_value<FT>(S, mi.y, h, status);
             em = rgb(tv.r * mf.z, tv.g * mf.z, tv.b * mf.z);
         }
-    } else if (mi.x == MAT_SPOT_LIGHT) {
+    } else if (!PLAIN && mi.x == MAT_SPOT_LIGHT) {
         // diffuse_spot_light::emitted (diffuse_spot_light.cuh:33-49).  Back face: RGBA(0,0,0,0) when
         // invisible, else RGBA(1,1,1,0) (both re-hit; the product with the attenuation adds 0 or 1);
         // outside the cone RGBA(1,1,1,1); inside texture * (intensity * pow(cos, falloff)).

@@ -445,7 +445,7 @@ __device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* it
             float a, b;
             const float4 q3 = __ldg(q + 3), q4 = __ldg(q + 4);
             bool hitl;
-            if (q4.w < 0.0f) {
+            if (!PLAIN && q4.w < 0.0f) {
                 // omni_light::hit / spot_light::hit (omni_light.cuh:55-83): the sphere quadratic, strict
                 const float4 sp = __ldg(q);
                 hitl = EXACT ? sphere_t_exact(sp, o, d, tmin, best_t, t) : sphere_t(sp, o, d, tmin, best_t, t);
@@ -849,7 +849,7 @@ __device__ __forceinline__ void finalize_prim(const DevScene& S, uint32_t kind, 
     case ITEM_LIGHT: {
         const float4* q = kind == ITEM_QUAD ? S.quad + 5 * (size_t)idx : S.light + 6 * (size_t)idx;
         float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3), q4 = __ldg(q + 4);
-        if (kind == ITEM_LIGHT && q4.w < 0.0f) {
+        if (!PLAIN && kind == ITEM_LIGHT && q4.w < 0.0f) {
             // omni / spot light (omni_light.cuh:85-102): outward normal (p - c) / radius; its texture is
             // a solid colour, so the sphere uv the reference also computes is not needed
             h.p = at(o, d, t);
@@ -879,7 +879,7 @@ __device__ __forceinline__ void finalize_prim(const DevScene& S, uint32_t kind, 
         float4 nn = __ldg(S.tri_n + idx);
         V3 normal = v3(nn.x, nn.y, nn.z);
         int sm = __float_as_int(a2.w);
-        if (sm >= 0) {
+        if (!PLAIN && sm >= 0) {
             // smooth: a*vn1 + b*vn2 + c*vn0 with the barycentrics of triangle::hit (triangle.cuh:171-175)
             V3 v0 = v3(a0.x, a0.y, a0.z), e1 = v3(a1.x, a1.y, a1.z), e2 = v3(a2.x, a2.y, a2.z);
             V3 pv = cross(d, e2);
@@ -894,7 +894,7 @@ __device__ __forceinline__ void finalize_prim(const DevScene& S, uint32_t kind, 
             normal = add(add(mul(bu, v3(__ldg(vn + 1))), mul(bv, v3(__ldg(vn + 2)))), mul(bc, v3(__ldg(vn))));
         }
         set_face_normal(h, d, normal);
-        if (S.tri_uv) {
+        if (!PLAIN && S.tri_uv) {
             tri_uv_at(S, idx, a0, a1, a2, h);
         } else {
             // no mesh has texture coordinates: get_triangle_uv over all-zero vertex uvs gives (0, 0)
@@ -978,6 +978,7 @@ __device__ __forceinline__ RGB texture_value(const DevScene& S, int tex, Hit& h,
             continue;
         }
         // image
+        if (PLAIN) break;
         if ((uint32_t)ti.w >= S.num_images) { status |= STATUS_BAD_TEXTURE; return rgb(0.f, 0.f, 0.f); }
         int4 im = __ldg(S.images + ti.w);
         int W = im.y, H = im.z;
@@ -1009,6 +1010,7 @@ __device__ __forceinline__ RGB background(const DevScene& S, V3 dir) {
         float b = 1.0f - a;
         return rgb(b * B.color[0] + a * B.top[0], b * B.color[1] + a * B.top[1], b * B.color[2] + a * B.top[2]);
     }
+    if (PLAIN) return rgb(0.f, 0.f, 0.f);
     double theta = acos((double)-ud.y);
     double phi = atan2((double)-ud.z, (double)ud.x) + 3.14159265358979323846;
     double uu = phi / (2.0 * 3.14159265358979323846);
@@ -1082,7 +1084,7 @@ __device__ __forceinline__ float light_pdf_value(const DevScene& S, uint32_t li,
     const float4* q = S.light + 6 * (size_t)li;
     float4 q0 = __ldg(q), q4 = __ldg(q + 4);
     float t, a, b;
-    if (q4.w < 0.0f) {
+    if (!PLAIN && q4.w < 0.0f) {
         if (!sphere_t(q0, o, v, 0.00001f, INFINITY, t)) return 0.0f;
         const float ctm = sqrtf(1.0f - q0.w * q0.w / lensq(sub(v3(q0.x, q0.y, q0.z), o)));
         const float solid_angle = 2.0f * 3.14159265358979323846f * (1.0f - ctm);

@@ -8,6 +8,8 @@ cudaError_t RTC_XP_FN(rtc_wf_one_clean)(WfOp op, const WfOneArgs& a, const WfBuf
     return wf_dispatch<true, 0, 2, WfOne>(op, a, B, L);
 }
 
+#if !RTC_PLAIN
 cudaError_t RTC_XP_FN(rtc_wf_table_clean)(WfOp op, const WfTableArgs& a, const WfBuffers& B, const WfLaunch& L) {
     return wf_dispatch<true, 0, 2, WfTable>(op, a, B, L);
 }
+#endif

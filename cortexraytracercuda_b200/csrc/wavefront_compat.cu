@@ -14,6 +14,8 @@ cudaError_t RTC_FLAVOR_FN(rtc_wf_one_compat)(WfOp op, const WfOneArgs& a, const 
     return wf_dispatch<false, RTC_FLAVOR, RTC_FLAVOR, WfOne>(op, a, B, L);
 }
 
+#if !RTC_PLAIN
 cudaError_t RTC_FLAVOR_FN(rtc_wf_table_compat)(WfOp op, const WfTableArgs& a, const WfBuffers& B, const WfLaunch& L) {
     return wf_dispatch<false, RTC_FLAVOR, RTC_FLAVOR, WfTable>(op, a, B, L);
 }
+#endif
