@@ -177,6 +177,11 @@ __device__ __forceinline__ bool planar_t(float4 q0, float4 q1, float4 q2, float4
 }
 
 // triangle::hit (triangle.cuh:130-160): Moller-Trumbore, |det| < 1e-6 rejected, inclusive bounds.
+//
+// FUSED: u + v of the last edge's test as one fused operation over u's product (FMA flavours only).  Left to
+// the compiler, the choice follows the code around it, and a ray through a shared edge (one in about 10^8 of
+// a mesh frame) takes the other triangle when it changes; so it is written out, per kernel (Edge).
+template <bool FUSED>
 __device__ __forceinline__ bool tri_t(float4 a0, float4 a1, float4 a2, V3 o, V3 d, float tmin, float tmax,
                                       float& t, float& bu, float& bv) {
     V3 v0 = v3(a0.x, a0.y, a0.z), e1 = v3(a1.x, a1.y, a1.z), e2 = v3(a2.x, a2.y, a2.z);
@@ -185,11 +190,12 @@ __device__ __forceinline__ bool tri_t(float4 a0, float4 a1, float4 a2, V3 o, V3 
     if (fabsf(det) < 0.000001f) return false;
     float inv_det = 1.0f / det;
     V3 tv = sub(o, v0);
-    float u = dot(tv, pv) * inv_det;
+    const float up = dot(tv, pv);
+    float u = up * inv_det;
     if (u < 0.0f || u > 1.0f) return false;
     V3 qv = cross(tv, e1);
     float v = dot(d, qv) * inv_det;
-    if (v < 0.0f || u + v > 1.0f) return false;
+    if (v < 0.0f || (FUSED ? __fmaf_rn(up, inv_det, v) : __fadd_rn(u, v)) > 1.0f) return false;
     float tt = dot(e2, qv) * inv_det;
     if (tt < tmin || tt > tmax) return false;
     t = tt;
@@ -355,10 +361,13 @@ struct XformRay {
     V3 o, d;
 };
 
+// Which triangles a kernel tests with the fused last edge (tri_t).
+enum Edge { EDGE_FUSED_MAIN = 1, EDGE_FUSED_XPRIM = 2 };
+
 // A leaf range of the xprim BVH, xprims [first, first + cnt) (leaf order is xprim order: item k of the list
 // is xprim k): transformed primitives and box faces, each tested on its object-space ray.  EXACT: clean
 // mode's double-precision sphere test.  Links and indices were checked when the scene was created.
-template <bool EXACT>
+template <bool EXACT, int EDGE>
 __device__ __forceinline__ void test_xprims(const DevScene& S, uint32_t first, uint32_t cnt, V3 o, V3 d, XformRay& xr,
                                             float tmin, float& best_t, uint32_t& best_item, TraceStats& st,
                                             uint32_t& status) {
@@ -387,7 +396,8 @@ __device__ __forceinline__ void test_xprims(const DevScene& S, uint32_t first, u
         case ITEM_TRI: {
             const float4* p = S.tri + 3 * (size_t)in;
             float bu, bv;
-            h = tri_t(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), xr.o, xr.d, tmin, best_t, t, bu, bv);
+            h = tri_t<(EDGE & EDGE_FUSED_XPRIM) != 0>(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), xr.o, xr.d, tmin, best_t, t,
+                                                       bu, bv);
         } break;
         case XPRIM_RECT: {
             float a, b;
@@ -410,7 +420,7 @@ constexpr uint32_t ITEMS_LISTED = 0xffffffffu;
 // consecutive words - one kind, indices in leaf order, which is how the primitives are packed - so that
 // the walk goes from the node straight to the primitive record; ITEMS_LISTED reads the list.  Words and
 // ranges were checked when the scene was created (rtc_api.cpp, check_tree), not per test.
-template <bool EXACT>
+template <bool EXACT, int EDGE>
 __device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* items, uint32_t first, uint32_t cnt, uint32_t word,
                                            V3 o, V3 d, float tmin, float& best_t, uint32_t& best_item,
                                            bool hide_invisible, TraceStats& st, uint32_t& status) {
@@ -423,7 +433,10 @@ __device__ __forceinline__ void test_items(const DevScene& S, const uint32_t* it
         case ITEM_TRI: {
             const float4* p = S.tri + 3 * (size_t)idx;
             float bu, bv;
-            if (tri_t(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), o, d, tmin, best_t, t, bu, bv)) { best_t = t; best_item = it; }
+            if (tri_t<(EDGE & EDGE_FUSED_MAIN) != 0>(ld_scene(p), ld_scene(p + 1), ld_scene(p + 2), o, d, tmin, best_t, t, bu, bv)) {
+                best_t = t;
+                best_item = it;
+            }
         } break;
         case ITEM_SPHERE: {
             const float4 sp = ld_scene(S.sph + idx);
@@ -500,7 +513,7 @@ __device__ __forceinline__ uint32_t octant_order(uint32_t h, uint32_t oct) {
 // child: a leaf is tested in place; for an inner child the rest of the group is pushed as one 32-bit
 // entry (node << 8 | mask) and the child's own group replaces it.  No sort, no distances on the stack:
 // at most one entry per level.
-template <bool EXACT>
+template <bool EXACT, int EDGE>
 __device__ __forceinline__ bool closest_hit8(const DevScene& S, V3 o, V3 d, V3 inv, V3 oi, float tmin, float tmax,
                                              bool hide_invisible, float& t_out, uint32_t& item_out,
                                              TraceStats& st, uint32_t& status) {
@@ -607,8 +620,8 @@ __device__ __forceinline__ bool closest_hit8(const DevScene& S, V3 o, V3 d, V3 i
         } else {
             const uint32_t first = (uint32_t)links.y + (lb & 31u), cnt = ((lb >> 5) & 3u) + 1u;
             if (first + cnt > S.num_items) { status |= STATUS_BAD_ITEM; break; }
-            test_items<EXACT>(S, S.items8, first, cnt, ITEMS_LISTED, o, d, tmin, best_t, best_item, hide_invisible, st,
-                              status);
+            test_items<EXACT, EDGE>(S, S.items8, first, cnt, ITEMS_LISTED, o, d, tmin, best_t, best_item, hide_invisible,
+                                    st, status);
         }
     }
     t_out = best_t;
@@ -640,7 +653,7 @@ __device__ __forceinline__ bool hit_leaves(int32_t cl, int32_t cr, uint32_t wl, 
 
 // The xprim BVH (binary, `xnodes`, leaves of xprims) against [tmin, best_t]: updates best_t / best_item and
 // returns whether any hit is held.  Same node layout and walk as the binary traversal below.
-template <bool EXACT>
+template <bool EXACT, int EDGE>
 __device__ __forceinline__ bool closest_hit_xprims(const DevScene& S, V3 o, V3 d, V3 inv, V3 oi, float tmin,
                                                 float& best_t, uint32_t& best_item, TraceStats& st,
                                                 uint32_t& status) {
@@ -658,7 +671,7 @@ __device__ __forceinline__ bool closest_hit_xprims(const DevScene& S, V3 o, V3 d
         bool hl = slab2(n0, n1, n2, inv, oi, tmin, best_t, tl, tr, hr);
         uint32_t first, cnt, word;
         if (hit_leaves(cl, cr, 0u, 0u, hl, hr, first, cnt, word))
-            test_xprims<EXACT>(S, first, cnt, o, d, xr, tmin, best_t, best_item, st, status);
+            test_xprims<EXACT, EDGE>(S, first, cnt, o, d, xr, tmin, best_t, best_item, st, status);
         if (hl && hr) {
             int32_t nearc = tl <= tr ? cl : cr;
             int32_t farc = tl <= tr ? cr : cl;
@@ -694,7 +707,7 @@ enum Walk { WALK_BINARY = 0, WALK_WIDE = 1, WALK_EITHER = 2 };   // EITHER: the 
 // entry distances on the stack to skip popped nodes behind the best hit (3% fewer visits, 3% slower), leaves
 // deferred until half a warp holds one (spheres 35 ms), idle lanes refilled from a pool of rays with the
 // tree in shared memory (36-40 ms).
-template <bool EXACT = false, int WALK = WALK_BINARY>
+template <bool EXACT = false, int WALK = WALK_BINARY, int EDGE = 0>
 __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float tmin, float tmax,
                                             bool hide_invisible, float& t_out, uint32_t& item_out,
                                             TraceStats& st, uint32_t& status) {
@@ -710,9 +723,9 @@ __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float
     if constexpr (WALK != WALK_BINARY) {
         if (WALK == WALK_WIDE || S.nodes8) {
             V3 oi8 = v3(o.x * inv.x, o.y * inv.y, o.z * inv.z);
-            bool h = closest_hit8<EXACT>(S, o, d, inv, oi8, tmin, tmax, hide_invisible, t_out, item_out, st, status);
+            bool h = closest_hit8<EXACT, EDGE>(S, o, d, inv, oi8, tmin, tmax, hide_invisible, t_out, item_out, st, status);
 #if RTC_XP
-            if (S.num_xnodes) h = closest_hit_xprims<EXACT>(S, o, d, inv, oi8, tmin, t_out, item_out, st, status);
+            if (S.num_xnodes) h = closest_hit_xprims<EXACT, EDGE>(S, o, d, inv, oi8, tmin, t_out, item_out, st, status);
 #endif
             return h;
         }
@@ -737,7 +750,7 @@ __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float
             bool hl = slab2(n0, n1, n2, inv, oi, tmin, best_t, tl, tr, hr);
             uint32_t first, cnt, word;
             if (hit_leaves(cl, cr, __float_as_uint(n3.z), __float_as_uint(n3.w), hl, hr, first, cnt, word))
-                test_items<EXACT>(S, S.items, first, cnt, word, o, d, tmin, best_t, best_item, hide_invisible, st, status);
+                test_items<EXACT, EDGE>(S, S.items, first, cnt, word, o, d, tmin, best_t, best_item, hide_invisible, st, status);
             if (hl && hr) {
                 int32_t nearc = tl <= tr ? cl : cr;
                 int32_t farc = tl <= tr ? cr : cl;
@@ -759,7 +772,7 @@ __device__ __forceinline__ bool closest_hit(const DevScene& S, V3 o, V3 d, float
         // transformed primitives and box faces live in their own BVH, walked after the first one against the
         // best hit so far; scenes without them skip it (and their traversal loop carries none of its registers)
 #if RTC_XP
-        if (S.num_xnodes) return closest_hit_xprims<EXACT>(S, o, d, inv, oi, tmin, t_out, item_out, st, status);
+        if (S.num_xnodes) return closest_hit_xprims<EXACT, EDGE>(S, o, d, inv, oi, tmin, t_out, item_out, st, status);
 #endif
         return best_item != 0xffffffffu;
     }
