@@ -1118,14 +1118,17 @@ struct WfTimer {
     }
 };
 
-// `xp`: the scene has transformed primitives or boxes (an xprim BVH), walked by the RTC_XP=1 kernels.
-rtc::WfOneFn wf_one_fn(const rtc_render_params* p, const rtc::DevScene& S) {
+// Scenes with transformed primitives or boxes (an xprim BVH) take the RTC_XP=1 kernels, plain scenes the
+// RTC_PLAIN=1 ones, except where the shade kernel takes chunks from a counter (`dynamic_shade`): in the plain
+// build that kernel rounds the dielectric's dot products differently (a 3.9 M triangle clean frame, 1920x1080,
+// 16 spp: 1.6% of the pixels), so it exists in the full build alone.
+rtc::WfOneFn wf_one_fn(const rtc_render_params* p, const rtc::DevScene& S, bool dynamic_shade) {
     static const rtc::WfOneFn fn[3][2][2] = {   // [clean, g++ flavour, nvcc flavour][xprims][plain]
         {{rtc_wf_one_clean, rtc_wf_one_clean_p}, {rtc_wf_one_clean_x, rtc_wf_one_clean_xp}},
         {{rtc_wf_one_compat_host, rtc_wf_one_compat_host_p}, {rtc_wf_one_compat_host_x, rtc_wf_one_compat_host_xp}},
         {{rtc_wf_one_compat_dev, rtc_wf_one_compat_dev_p}, {rtc_wf_one_compat_dev_x, rtc_wf_one_compat_dev_xp}}};
     const int m = p->mode == RTC_MODE_CLEAN ? 0 : p->draw_order == RTC_DRAW_ORDER_HOST ? 1 : 2;
-    return fn[m][S.num_xnodes != 0][S.plain != 0];
+    return fn[m][S.num_xnodes != 0][S.plain != 0 && !dynamic_shade];
 }
 
 rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const WfBuffers& B, uint32_t* d_status,
@@ -1140,7 +1143,10 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     DevParams P = dev_params(p);
     P.rgb8 = d_rgb8;   // quantised output written as each pixel finishes
     const bool clean = p->mode == RTC_MODE_CLEAN;
-    const WfOneFn fn = wf_one_fn(p, S);
+    // scenes whose walks are long and uneven: see the launches below
+    const bool large = S.num_items >= (1u << 20);
+    const bool dynamic_extend = rtc_dynamic_chunks(large), dynamic_shade = rtc_dynamic_chunks(large && clean);
+    const WfOneFn fn = wf_one_fn(p, S, dynamic_shade);
     WfOneArgs J;
     J.S = S;
     J.P = P;
@@ -1187,8 +1193,6 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     // resident wave; the long grid costs it 5-15%); the counter costs it more than it balances (same frame: 10.1
     // against 8.3 ms), but clean mode keeps it in those scenes, where the two kernels round a refraction
     // differently in the last bit.
-    const bool large = S.num_items >= (1u << 20);
-    const bool dynamic_extend = rtc_dynamic_chunks(large), dynamic_shade = rtc_dynamic_chunks(large && clean);
     // long-chain split: at iteration `split_at` (0: never), slots predicted to need more than
     // `split_thr` further iterations move to the drain kernel, running beside the bulk iterations
     uint64_t split_at = 0;

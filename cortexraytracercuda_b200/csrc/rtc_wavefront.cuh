@@ -1065,7 +1065,10 @@ cudaError_t wf_dispatch(WfOp op, const A& args, const WfBuffers& B, const WfLaun
         if (L.dynamic) return wf_launch_extend<FLAVOR, J, true>(jobs, B, L, blk, c);
         return wf_launch_extend<FLAVOR, J, false>(jobs, B, L, blk, c);
     case WF_OP_SHADE:
-        if (L.dynamic) return wf_launch_shade<CLEAN, ORDER, J, true>(jobs, B, L, blk, c);
+        if (L.dynamic) {   // not in the plain build (rtc_api.cpp, wf_one_fn)
+            if constexpr (PLAIN) return cudaErrorInvalidValue;
+            else return wf_launch_shade<CLEAN, ORDER, J, true>(jobs, B, L, blk, c);
+        }
         return wf_launch_shade<CLEAN, ORDER, J, false>(jobs, B, L, blk, c);
     case WF_OP_FINISH:
         if (L.drain_every > 0) {
