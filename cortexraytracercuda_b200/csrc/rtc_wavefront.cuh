@@ -485,14 +485,21 @@ __global__ void __launch_bounds__(128) wf_admit(WfTable J, WfBuffers B, WfIter w
     if (status) atomicOr(status_word, status);
 }
 
-// Which triangles the extend kernel tests with the fused last edge (tri_t), by flavour, job source and node
-// layout: what the compiler chose for each before it was written out, so that images stay as they were.  The
-// other kernels fuse none, except wf_bounces, which stands in for the binary extend kernel of one image.
-__host__ __device__ constexpr int extend_edge(int flavor, bool one, bool wide) {
+// Which triangles the extend kernel tests with the fused last edge (tri_t), by flavour, job source, node layout
+// and instrumentation: what the compiler chose for each before it was written out, so that images stay as they
+// were.  The other kernels fuse none, except wf_bounces, which stands in for the binary extend of one image.
+__host__ __device__ constexpr int extend_edge(int flavor, bool one, bool wide, bool count) {
     if (flavor == 1) return 0;   // no contraction
     const bool clean = flavor == 2, xp = RTC_XP != 0;
-    const bool main = one ? wide && (clean || xp) : clean || wide || !xp;
-    const bool xprim = !one || wide || !clean;
+    bool main = true, xprim = true;
+    if (clean && one) {
+        main = count ? !wide && !xp : wide;
+        xprim = !count && wide;
+    } else if (one) {
+        main = count ? wide || xp : wide && xp;
+    } else if (!clean) {
+        main = wide || !xp || count;
+    }
     return (main ? EDGE_FUSED_MAIN : 0) | (xprim ? EDGE_FUSED_XPRIM : 0);
 }
 
@@ -527,7 +534,7 @@ __global__ void RTC_EXTEND_BOUNDS wf_extend(J jobs, WfBuffers B, WfIter w, unsig
             constexpr int WALK = !WIDE ? WALK_BINARY : ONE ? WALK_WIDE : WALK_EITHER;
             uint32_t* sh = wf_sec(B, slot, SEC_SHADE);
             const float tmin = ray_tmin<FLAVOR == 2>(R, [&] { return ld_word(sh + 6); });
-            bool h = closest_hit<FLAVOR == 2, WALK, extend_edge(FLAVOR, ONE, WIDE)>(
+            bool h = closest_hit<FLAVOR == 2, WALK, extend_edge(FLAVOR, ONE, WIDE, COUNT)>(
                 jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), tmin, 3.402823466e+38f,
                 wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t, item, st, status);
             st_hit(sh, t, h ? item : 0xffffffffu);
@@ -745,7 +752,7 @@ __global__ void __launch_bounds__(WF_BOUNCES_BLOCK, 20) wf_bounces(J jobs, WfBuf
                 const uint32_t job = wf_job(mw);
                 float t;
                 uint32_t item;
-                const bool h = closest_hit<CLEAN, WALK_BINARY, extend_edge(CLEAN ? 2 : ORDER, true, false)>(
+                const bool h = closest_hit<CLEAN, WALK_BINARY, extend_edge(CLEAN ? 2 : ORDER, true, false, false)>(
                     jobs.scene(job), sec_v3(R, 0), sec_v3(R, 3), ray_tmin<CLEAN>(R, [&] { return SH.w[6]; }),
                     3.402823466e+38f, wf_depth(mw) == (uint32_t)jobs.params(job).max_depth, t, item, st, status);
                 live = wf_step<CLEAN, ORDER, true>(jobs, win, B, slot, R, SH, PX, t, h ? item : 0xffffffffu, pc, st, paths,
