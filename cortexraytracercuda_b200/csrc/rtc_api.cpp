@@ -69,7 +69,7 @@ extern "C" rtc_status rtc_context_create(int device, rtc_context** out) {
     c->device = device;
     c->num_sms = prop.multiProcessorCount;
     cudaError_t e1 = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-    cudaError_t e2 = cudaMalloc(&c->d_status, sizeof(uint32_t));
+    cudaError_t e2 = cudaMalloc(&c->d_status, 2 * sizeof(uint32_t));
     cudaError_t e3 = cudaMalloc(&c->d_counters, CNT_N * sizeof(unsigned long long));
     if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess) {
         cudaError_t e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
@@ -1345,6 +1345,14 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     return RTC_OK;
 }
 
+// Orders `st` after the context's last wavefront render, which may still be running on another stream: renders of
+// a context share its path state, queues and status word.  The end of that render is waited for on whatever
+// stream this is (a stream's handle does not tell whether it is the same stream: handles are reused, and
+// cudaStreamPerThread names one stream per thread); on the same stream it is already in order and costs nothing.
+cudaError_t after_last_render(rtc_context* c, cudaStream_t st) {
+    return c->phase_ev[2] ? cudaStreamWaitEvent(st, c->phase_ev[2], 0) : cudaSuccess;
+}
+
 rtc_status launch_wavefront(rtc_context* c, const rtc_scene* s, const rtc_render_params* p, float4* d_out,
                             unsigned long long* d_counters, cudaStream_t st, uint8_t* d_rgb8) {
     const int64_t units = (int64_t)p->width * p->height * dev_params(p).groups;
@@ -1352,6 +1360,7 @@ rtc_status launch_wavefront(rtc_context* c, const rtc_scene* s, const rtc_render
     WfBuffers B;
     rtc_status r = ensure_wavefront(c, slots, B);
     if (r != RTC_OK) return r;
+    RTC_CUDA(after_last_render(c, st));
     const size_t gbytes = rtc_group_bytes(p);
     if (gbytes > c->groups_cap) {
         cudaFree(c->d_groups);
@@ -1373,7 +1382,12 @@ rtc_status launch_wavefront(rtc_context* c, const rtc_scene* s, const rtc_render
     const bool timed = (p->flags & RTC_FLAG_KERNEL_TIMING) != 0;
     r = run_wavefront(rtc_scene_view(s, p), p, B, c->d_status, d_out, d_counters, st, c->num_sms, poll,
                       c->phase_ev, run, timed ? &timer : nullptr, c->d_groups, d_rgb8);
-    if (r != RTC_OK) return r;
+    if (r != RTC_OK) {
+        // no end was recorded for the next render to wait for: wait here for what was queued
+        cudaStreamSynchronize(st);
+        cudaStreamSynchronize(c->stream_long);
+        return r;
+    }
     c->kev_ext = c->kev_shade = 0;
     c->kev_pairs.clear();
     if (timed) {
@@ -1433,9 +1447,9 @@ rtc_status launch(rtc_context* c, const rtc_scene* s, const rtc_render_params* p
     return RTC_OK;
 }
 
-rtc_status read_status(rtc_context* c) {
+rtc_status read_status(rtc_context* c, const uint32_t* d_status) {
     uint32_t st = 0;
-    RTC_CUDA(cudaMemcpyAsync(&st, c->d_status, 4, cudaMemcpyDeviceToHost, c->stream));
+    RTC_CUDA(cudaMemcpyAsync(&st, d_status, 4, cudaMemcpyDeviceToHost, c->stream));
     RTC_CUDA(cudaStreamSynchronize(c->stream));
     if (st) {
         char buf[128];
@@ -1470,6 +1484,7 @@ extern "C" rtc_status rtc_render(rtc_context* c, const rtc_scene* s, const rtc_r
         RTC_CUDA(cudaMalloc(&c->d_rgb8, npix * 3));
         c->rgb8_cap = npix * 3;
     }
+    RTC_CUDA(after_last_render(c, c->stream));   // it may still write the status word
     RTC_CUDA(cudaMemsetAsync(c->d_status, 0, 4, c->stream));
     r = launch(c, s, p, c->d_out, nullptr, c->stream, rgb8 ? c->d_rgb8 : nullptr);
     if (r != RTC_OK) return r;
@@ -1477,7 +1492,7 @@ extern "C" rtc_status rtc_render(rtc_context* c, const rtc_scene* s, const rtc_r
     if (radiance_sum)
         RTC_CUDA(cudaMemcpyAsync(radiance_sum, c->d_out, npix * sizeof(float4), cudaMemcpyDeviceToHost, c->stream));
     RTC_CUDA(cudaStreamSynchronize(c->stream));
-    return read_status(c);
+    return read_status(c, c->d_status);
 }
 
 extern "C" rtc_status rtc_render_device(rtc_context* c, const rtc_scene* s, const rtc_render_params* p,
@@ -1487,6 +1502,7 @@ extern "C" rtc_status rtc_render_device(rtc_context* c, const rtc_scene* s, cons
     if (((uintptr_t)d_radiance_sum & 15u) != 0) return fail(RTC_ERR_INVALID_ARGUMENT, "radiance buffer must be 16-byte aligned");
     rtc_status r = check_params(p);
     if (r != RTC_OK) return r;
+    std::lock_guard<std::mutex> lk(c->mu);
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     RtcDeviceScope dev(c->device);
     RTC_CUDA(dev.error());
@@ -1495,6 +1511,7 @@ extern "C" rtc_status rtc_render_device(rtc_context* c, const rtc_scene* s, cons
 
 extern "C" rtc_status rtc_get_render_stats(rtc_context* c, rtc_render_stats* out) {
     if (!c || !out) return fail(RTC_ERR_INVALID_ARGUMENT, "null argument");
+    std::lock_guard<std::mutex> lk(c->mu);
     *out = c->last;
     if (c->last_timed) {
         RTC_CUDA(cudaEventSynchronize(c->phase_ev[2]));
@@ -1547,20 +1564,21 @@ extern "C" rtc_status rtc_trace_closest_ex(rtc_context* c, const rtc_scene* s, c
     float* d_rays = (float*)block;
     int32_t* d_prim = (int32_t*)((uint8_t*)block + rays_bytes);
     float* d_t = (float*)(d_prim + n);
+    uint32_t* d_status = c->d_status + 1;   // not the renders': one may be running on another stream
     cudaError_t e = cudaMemcpyAsync(d_rays, rays, rays_bytes, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, 4, c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_status, 0, 4, c->stream);
     rtc_render_params vp{};
     vp.flags = flags;
     const DevScene SV = rtc_scene_view(s, &vp);
     auto tfn = SV.num_xnodes ? rtc_launch_trace_closest_x : rtc_launch_trace_closest;
-    if (e == cudaSuccess) e = tfn(SV, d_rays, n, depth, max_depth, d_prim, d_t, c->d_status, c->stream);
+    if (e == cudaSuccess) e = tfn(SV, d_rays, n, depth, max_depth, d_prim, d_t, d_status, c->stream);
     if (e == cudaSuccess && prim) e = cudaMemcpyAsync(prim, d_prim, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess && t) e = cudaMemcpyAsync(t, d_t, (size_t)n * 4, cudaMemcpyDeviceToHost, c->stream);
     const cudaError_t e2 = cudaStreamSynchronize(c->stream);   // also before the block is freed or reused
     if (e == cudaSuccess) e = e2;
     if (block != c->d_trace) cudaFree(block);
     if (e != cudaSuccess) return cuda_fail(e, "trace_closest");
-    return read_status(c);
+    return read_status(c, d_status);
 }
 
 // ---------------------------------------------------------------------------------------------------

@@ -16,7 +16,7 @@
 struct rtc_context {
     int device = 0;
     cudaStream_t stream = nullptr;
-    uint32_t* d_status = nullptr;
+    uint32_t* d_status = nullptr;     // kernel status words: [0] renders, [1] rtc_trace_closest
     unsigned long long* d_counters = nullptr;
     float4* d_out = nullptr;
     size_t out_cap = 0;         // float4 elements
@@ -34,7 +34,8 @@ struct rtc_context {
     size_t trace_cap = 0;
     uint32_t* h_poll = nullptr;       // pinned: queue sizes read back between batches
     cudaEvent_t poll_ev[2] = {nullptr, nullptr};
-    cudaEvent_t phase_ev[3] = {nullptr, nullptr, nullptr};   // render start, drain start, render end
+    cudaEvent_t phase_ev[3] = {nullptr, nullptr, nullptr};   // render start, drain start, render end (which the
+                                                             // next render waits for: after_last_render)
     cudaStream_t stream_long = nullptr;    // the long-chain drain kernel, beside the bulk iterations
     cudaEvent_t split_ev[2] = {nullptr, nullptr};
     rtc_render_stats last{};

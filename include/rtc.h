@@ -443,7 +443,10 @@ rtc_status rtc_render(rtc_context* ctx, const rtc_scene* scene, const rtc_render
  * tests, then the wavefront extend kernel's own rays, node visits and primitive tests, one unused.  The megakernel engine
  * returns without waiting for the GPU; the wavefront engine polls its queue counter between batches
  * of iterations (a frame of fewer than 512 work units per SM is queued without a poll).  The last
- * kernels may still run when it returns, in order on `stream`.  A stream under capture is refused. */
+ * kernels may still run when it returns, in order on `stream`.  Renders of one context share its scratch
+ * memory: on the wavefront engine, a render given another stream than the one before first waits for that
+ * one, on the device.  Calls from several threads are taken one after another.  A stream under capture is
+ * refused. */
 rtc_status rtc_render_device(rtc_context* ctx, const rtc_scene* scene, const rtc_render_params* params,
                              float* d_radiance_sum, uint8_t* d_rgb8, unsigned long long* d_counters,
                              void* stream);
