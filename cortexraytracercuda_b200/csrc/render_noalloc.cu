@@ -14,7 +14,8 @@
 //   * one path slot per pixel, so one call renders at most RTC_NOALLOC_MAX_PIXELS (508,376) pixels
 //     and rejects larger images with RTC_ERR_INVALID_ARGUMENT before touching the GPU;
 //   * the first call on a device looks up the array's device address (cudaGetSymbolAddress, once per
-//     device, with that device current); make that first call before any stream capture;
+//     device, with that device current); make that first call before any stream capture; a stream
+//     under capture is refused before anything is queued;
 //   * every call shares the array: the counters and the status word are cleared at the start of each
 //     call, the rest is fully rewritten; calls that overlap on the GPU (two streams, two threads)
 //     race on it;
@@ -79,10 +80,12 @@ extern "C" rtc_status rtc_render_noalloc(const rtc_scene* scene, const rtc_rende
     RtcDeviceScope dev(device);   // the caller's current device is restored on return
     cudaError_t e = dev.error();
     if (e != cudaSuccess) return rtc_set_error(RTC_ERR_CUDA, cudaGetErrorString(e));
+    cudaStream_t st = (cudaStream_t)stream;
+    r = rtc_refuse_capture(st);
+    if (r != RTC_OK) return r;
     void* base = nullptr;
     r = scratch_address(device, &base);
     if (r != RTC_OK) return r;
-    cudaStream_t st = (cudaStream_t)stream;
     uint32_t* d_status = (uint32_t*)base;
     rtc::WfBuffers B;
     if (NOALLOC_HEADER_BYTES + rtc_carve_wavefront((uint8_t*)base + NOALLOC_HEADER_BYTES, (uint32_t)npix, B) >

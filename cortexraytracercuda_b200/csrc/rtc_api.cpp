@@ -1135,11 +1135,6 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
                          float4* d_out, unsigned long long* d_counters, cudaStream_t st, int num_sms,
                          const WfPoller& poll, cudaEvent_t* phase, WfRun& run, WfTimer* timer = nullptr,
                          void* groups = nullptr, uint8_t* d_rgb8 = nullptr) {
-    // A render shares its context's scratch (or the static array) with the renders after it and polls its
-    // queue, so it cannot be captured; a frame short enough to need no poll is refused like any other.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    RTC_CUDA(cudaStreamIsCapturing(st, &capturing));
-    if (capturing != cudaStreamCaptureStatusNone) return fail(RTC_ERR_CUDA, "a render cannot be captured into a graph");
     DevParams P = dev_params(p);
     P.rgb8 = d_rgb8;   // quantised output written as each pixel finishes
     const bool clean = p->mode == RTC_MODE_CLEAN;
@@ -1413,6 +1408,12 @@ size_t rtc_carve_wavefront(void* base, uint32_t slots, WfBuffers& B) { return ca
 rtc_status rtc_set_error(rtc_status s, const char* msg) { return fail(s, msg); }
 rtc_status rtc_check_render_params(const rtc_render_params* p) { return check_params(p); }
 int rtc_scene_device(const rtc_scene* s) { return s->device; }
+rtc_status rtc_refuse_capture(cudaStream_t st) {
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    RTC_CUDA(cudaStreamIsCapturing(st, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return fail(RTC_ERR_CUDA, "a render cannot be captured into a graph");
+    return RTC_OK;
+}
 rtc_status rtc_run_wavefront_sync(const rtc_scene* s, const rtc_render_params* p, const WfBuffers& B,
                                   uint32_t* d_status, float4* d_out, cudaStream_t st) {
     int dev = 0, sms = 148;
@@ -1506,6 +1507,10 @@ extern "C" rtc_status rtc_render_device(rtc_context* c, const rtc_scene* s, cons
     cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
     RtcDeviceScope dev(c->device);
     RTC_CUDA(dev.error());
+    if (p->engine != RTC_ENGINE_MEGAKERNEL) {
+        r = rtc_refuse_capture(st);
+        if (r != RTC_OK) return r;
+    }
     return launch(c, s, p, (float4*)d_radiance_sum, d_counters, st, d_rgb8);
 }
 

@@ -39,6 +39,9 @@ size_t rtc_carve_wavefront(void* base, uint32_t slots, rtc::WfBuffers& B);
 // records an error message for rtc_last_error_string() and returns `s`
 rtc_status rtc_set_error(rtc_status s, const char* msg);
 rtc_status rtc_check_render_params(const rtc_render_params* p);
+// an error when `st` is being captured: a wavefront render shares scratch memory with the renders after it and
+// polls its queue, so it cannot be part of a graph
+rtc_status rtc_refuse_capture(cudaStream_t st);
 // device-side view of a scene, and the per-launch parameters of a render
 const rtc::DevScene& rtc_scene_dev(const rtc_scene* s);
 // the device view a render uses: the 8-wide nodes only when the params ask for RTC_FLAG_WIDE_BVH

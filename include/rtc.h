@@ -445,8 +445,9 @@ rtc_status rtc_render(rtc_context* ctx, const rtc_scene* scene, const rtc_render
  * of iterations (a frame of fewer than 512 work units per SM is queued without a poll).  The last
  * kernels may still run when it returns, in order on `stream`.  Renders of one context share its scratch
  * memory: on the wavefront engine, a render given another stream than the one before first waits for that
- * one, on the device.  Calls from several threads are taken one after another.  A stream under capture is
- * refused. */
+ * one, on the device.  Calls from several threads are taken one after another.  The wavefront engine
+ * refuses a stream under capture (RTC_ERR_CUDA, before it allocates or queues anything: the capture goes
+ * on); the megakernel engine's launch may be captured. */
 rtc_status rtc_render_device(rtc_context* ctx, const rtc_scene* scene, const rtc_render_params* params,
                              float* d_radiance_sum, uint8_t* d_rgb8, unsigned long long* d_counters,
                              void* stream);
@@ -479,7 +480,7 @@ rtc_status rtc_get_render_stats(rtc_context* ctx, rtc_render_stats* stats);
  * and needs no context: the scene (already on its device) and the 16-byte aligned device output
  * (width*height float4, frame-buffer order) come from the caller; `stream` may be NULL (legacy
  * stream).  The first call on a device looks up the array's address; make it before any stream
- * capture.  All calls share the array, so calls that overlap on the GPU race.  Returns when the frame
+ * capture.  A stream under capture is refused before anything is queued.  All calls share the array, so calls that overlap on the GPU race.  Returns when the frame
  * is complete; a call that fails part-way first waits for its queued kernels.  It always runs the
  * wavefront engine untimed (params->engine and RTC_FLAG_KERNEL_TIMING are ignored), and the calling
  * thread's current device is unchanged on return. */
