@@ -1172,11 +1172,9 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
     // drain threshold: below this many queued slots the finish kernel takes over
     uint32_t drain = (uint32_t)num_sms * 512u;
     if (const char* ev = std::getenv("RTC_WF_DRAIN")) drain = (uint32_t)std::strtoul(ev, nullptr, 10);
-    // Drain kernel: one thread per slot, or the compacting drain, whose live slots are repacked into full
-    // warps every 2 bounce steps, for scenes with transformed primitives: their two walks and transforms
-    // make a bounce instruction-bound, where packing pays (5-15% of a frame at 16 or more spp); elsewhere
-    // the longest chains' latency bounds the drain and repacking costs 2-50% (wf_finish, wf_finish_packed).
-    L.drain_every = rtc_drain_every(S.num_xnodes ? 2 : 0);
+    // Drain kernel: one thread per slot.  The compacting drain (wf_finish_packed) is left to RTC_WF_DRAIN_EVERY:
+    // no rule on what a scene contains separates where it pays (see there).
+    L.drain_every = rtc_drain_every(0);
     // Work distribution of the iteration kernels.  Extend: a grid as long as the queue can be, up to four
     // resident waves (32 blocks per SM), so that the block scheduler balances uneven walks and a launch does
     // not end on a half-empty round of one wave's stride (one wave: spheres frame 54.7 against 53.7 ms, an

@@ -922,11 +922,13 @@ __global__ void __launch_bounds__(WF_FINISH_BLOCK, 16) wf_finish(J jobs, WfBuffe
 // Compacting drain.  Every `every` steps the live slots of a 256-thread block move, through shared memory,
 // to the block's lowest threads: the live chains stay packed into full warps, and the warps left without a
 // slot wait at the block barrier without issuing.  Each slot computes exactly what the drain above computes
-// for it (the same step in the same order); only which thread runs it changes.  It pays where a bounce is
-// bound by instructions rather than by the latency of the longest chain: scenes with transformed primitives
-// (the second walk and the transforms; 333x251, 32 spp, clean: drain 5.5 -> 4.7 ms; 5-15% of the frame at
-// 30-235 K pixels and 16 or more spp).  Elsewhere the barriers and the dense tail cost: 2-8% of the frame on
-// small scenes, 25-50% on triangle meshes.
+// for it (the same step in the same order); only which thread runs it changes.  Off unless RTC_WF_DRAIN_EVERY
+// asks for it.  Every 2 steps against the drain above, frames of 24 scenes with transformed primitives, 7 to 300 K
+// pixels, 4 to 32 spp: it gains up to 13% where a few hundred primitives meet long chains (Cornell room with
+// transformed boxes 333x251, 32 spp, clean: 6.92 against 7.16 ms; 328 primitives with lights and one box: 3.57
+// against 3.98) and costs up to 60% elsewhere: 40 boxes in the open at 200x150 4.45 against 3.30 ms, 5,120
+// triangles 4.83 against 3.70, 1.31 M triangles and one box 300x200 11.6 against 7.7, 1920x1080 66.4 against 62.6.
+// With sample groups, whose chains are short, the two are equal.  Scenes without transformed primitives lose 2-50%.
 //
 // A block takes the queue entries b, b + G, b + 2G, ... (G blocks), so pixels that sit together in the
 // queue - neighbours, with similar chains - spread over all SMs; entries past G x WF_DRAIN_BLOCK are
