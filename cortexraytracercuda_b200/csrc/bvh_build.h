@@ -34,7 +34,8 @@ struct BvhOutput {
 };
 
 // Returns false (with a message) if the tree would not fit the traversal stack or the item encoding.
-// `wide`: also make the 8-wide nodes.
+// `wide`: also make the 8-wide nodes.  `threads`: at most this many threads build at once, the caller's and, in
+// the whole process, those added to it (0: four per hardware thread).  The tree does not depend on it.
 bool build_bvh(const BvhInput& in, int max_leaf, int threads, BvhOutput& out, const char** err, bool wide = true);
 
 // Merges subtrees of at most `max_leaf` primitives into single leaves where the SAH cost favours it
