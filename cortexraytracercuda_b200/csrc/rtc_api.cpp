@@ -1406,6 +1406,7 @@ size_t rtc_carve_wavefront(void* base, uint32_t slots, WfBuffers& B) { return ca
 rtc_status rtc_set_error(rtc_status s, const char* msg) { return fail(s, msg); }
 rtc_status rtc_check_render_params(const rtc_render_params* p) { return check_params(p); }
 int rtc_scene_device(const rtc_scene* s) { return s->device; }
+extern "C" int rtc_scene_plain(const rtc_scene* s) { return s && s->dev.plain ? 1 : 0; }
 rtc_status rtc_refuse_capture(cudaStream_t st) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     RTC_CUDA(cudaStreamIsCapturing(st, &capturing));

@@ -62,6 +62,8 @@ void rtc_carve_groups(void* base, const rtc_render_params* p, float4** part, uin
 // perspective_camera::initialize; false for a degenerate camera
 bool rtc_make_camera(const rtc_camera& c, rtc::DevCamera& out);
 int rtc_scene_device(const rtc_scene* s);
+// whether a scene's single images take the RTC_PLAIN=1 kernels (DevScene::plain); C linkage for the tests
+extern "C" int rtc_scene_plain(const rtc_scene* s);
 // runs the wavefront engine on caller-provided buffers with synchronous queue polling: no device or
 // pinned allocations, no events
 rtc_status rtc_run_wavefront_sync(const rtc_scene* s, const rtc_render_params* p, const rtc::WfBuffers& B,
