@@ -188,9 +188,30 @@ struct PathCounters {
     uint32_t rays, nodes, prims;
 };
 
+// A dielectric's dot(n, d) and its scattered direction, reflect or refract (rtc_math.cuh).  The FMA flavours'
+// compiler rounds that dot product in one of several ways, by the kernel around it.  COUNTED writes out the way
+// of clean mode's instrumented shade kernel of one image, so that its images do not move with that kernel's code.
+__device__ __forceinline__ float glass_dot(V3 n, V3 d) {
+    return __fadd_rn(__fmaf_rn(n.x, d.x, __fmul_rn(n.y, d.y)), __fmul_rn(n.z, d.z));
+}
+template <bool COUNTED>
+__device__ __forceinline__ V3 glass_direction(V3 d, V3 n, bool reflected, float eta) {
+    if constexpr (!COUNTED) {
+        return reflected ? reflect(d, n) : refract(d, n, eta);
+    } else {
+        const float dn = glass_dot(n, d);
+        if (reflected) return sub(d, mul(mul(n, dn), 2.0f));
+        const float k = __fmaf_rn(-__fmul_rn(eta, eta), __fmaf_rn(-dn, dn, 1.0f), 1.0f);
+        if (!(k >= 0.0f)) return v3(0.0f, 0.0f, 0.0f);
+        const float s = __fmaf_rn(eta, dn, sqrtf(k));
+        return v3(__fmaf_rn(eta, d.x, -__fmul_rn(s, n.x)), __fmaf_rn(eta, d.y, -__fmul_rn(s, n.y)),
+                  __fmaf_rn(eta, d.z, -__fmul_rn(s, n.z)));
+    }
+}
+
 // material::scatter of the hit material (metal, dielectric or lambertian; lights are handled by the
 // caller): updates the attenuation and turns `r` into the scattered ray (camera.cuh:185-225).
-template <bool CLEAN, int ORDER, class R>
+template <bool CLEAN, int ORDER, bool COUNTED_GLASS = false, class R>
 __device__ __forceinline__ void scatter_bounce(const DevScene& S, Ray& r, Hit& h, int4 mi, float4 mf, RGB& att,
                                                R& rng, uint32_t& status) {
     constexpr bool FT = CLEAN || ORDER == 0;   // float trig in the nvcc flavour and in clean mode
@@ -210,7 +231,7 @@ __device__ __forceinline__ void scatter_bounce(const DevScene& S, Ray& r, Hit& h
         // dielectric::scatter (dielectric.cuh:32-52) with Schlick (dielectric.cuh:57-63)
         float ratio = h.front ? (1.0f / mf.y) : mf.y;
         V3 ud = unit(r.d);
-        float ct = dot(neg(ud), h.n);
+        float ct = COUNTED_GLASS ? -glass_dot(h.n, ud) : dot(neg(ud), h.n);
         float cos_theta = ct < 1.0f ? ct : 1.0f;
         float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
         bool cannot_refract = ratio * sin_theta > 1.0f;
@@ -225,7 +246,7 @@ __device__ __forceinline__ void scatter_bounce(const DevScene& S, Ray& r, Hit& h
             float refl = r0 + (1.0f - r0) * p5;
             do_reflect = refl > rng.uniform();
         }
-        r.d = do_reflect ? reflect(ud, h.n) : refract(ud, h.n, ratio);
+        r.d = glass_direction<COUNTED_GLASS>(ud, h.n, do_reflect, ratio);
         r.o = scatter_origin<CLEAN>(h.p, h.n, r.d);
         return;   // attenuation (1,1,1)
     }
@@ -340,7 +361,7 @@ __device__ __forceinline__ RGB emitted(const DevScene& S, const Ray& r, Hit& h, 
 // With `rehit`, a miss or a light leaves the path ending on the light (rec keeps the light's material,
 // whose scatter returns false), anything else scatters with no emission added - exactly camera.cuh:177-190.
 enum BounceOut { BOUNCE_END = 0, BOUNCE_NEXT = 1, BOUNCE_REHIT = 2 };
-template <bool CLEAN, int ORDER, class R>
+template <bool CLEAN, int ORDER, bool COUNTED_GLASS = false, class R>
 __device__ __forceinline__ int shade_bounce_deferred(const DevScene& S, Ray& r, bool hit, float t, uint32_t item,
                                                      bool rehit, RGB& result, RGB& att, R& rng, uint32_t& status,
                                                      float& rehit_tmin) {
@@ -370,7 +391,7 @@ __device__ __forceinline__ int shade_bounce_deferred(const DevScene& S, Ray& r, 
         }
     }
     if (is_light_material(mi.x)) return BOUNCE_END;
-    scatter_bounce<CLEAN, ORDER>(S, r, h, mi, mf, att, rng, status);
+    scatter_bounce<CLEAN, ORDER, COUNTED_GLASS>(S, r, h, mi, mf, att, rng, status);
     return BOUNCE_NEXT;
 }
 

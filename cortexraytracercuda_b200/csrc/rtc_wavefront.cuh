@@ -563,7 +563,7 @@ __global__ void RTC_EXTEND_BOUNDS wf_extend(J jobs, WfBuffers B, WfIter w, unsig
 
 // One shade step of a slot whose current ray has been traced: shade_bounce_deferred, then the slot's
 // bookkeeping (next bounce / next sample / next pixel).  Returns true while the slot has a ray to trace.
-template <bool CLEAN, int ORDER, bool OWN = false, class J>
+template <bool CLEAN, int ORDER, bool OWN = false, bool COUNTED_GLASS = false, class J>
 __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, const WfBuffers& B, uint32_t slot,
                                         const Sec& R, const Sec& SH, const Sec& PX, float t, uint32_t item,
                                         PathCounters& pc, TraceStats& st, uint32_t& paths, uint32_t& status) {
@@ -582,8 +582,9 @@ __device__ __forceinline__ bool wf_step(const J& jobs, const WfWindow& win, cons
     rng_load<CLEAN>(R, PX, rng);   // of the pixel sector only clean mode's stream is read before the sample ends
     uint32_t depth = wf_depth(R.w[7]);
     float rehit_tmin = 0.0f;
-    const int out = shade_bounce_deferred<CLEAN, ORDER>(S, r, item != 0xffffffffu, t, item, ray_rehit<CLEAN>(R), acc,
-                                                        att, rng, status, rehit_tmin);
+    const int out = shade_bounce_deferred<CLEAN, ORDER, COUNTED_GLASS>(S, r, item != 0xffffffffu, t, item,
+                                                                       ray_rehit<CLEAN>(R), acc, att, rng, status,
+                                                                       rehit_tmin);
     uint32_t* rec_ray = wf_sec(B, slot, SEC_RAY);
     uint32_t* rec_shade = wf_sec(B, slot, SEC_SHADE);
     uint32_t* rec_px = wf_sec(B, slot, SEC_PIXEL);
@@ -680,7 +681,9 @@ __device__ __forceinline__ void wf_shade_pass(const J& jobs, const WfBuffers& B,
             const Sec SH = ld_sec(wf_sec(B, slot, SEC_SHADE));
             Sec PX{};
             if constexpr (CLEAN) PX = ld_sec(wf_sec(B, slot, SEC_PIXEL));
-            live = wf_step<CLEAN, ORDER>(jobs, win, B, slot, R, SH, PX, sec_f(SH, 6), SH.w[7], pc, st, paths, status);
+            constexpr bool COUNTED_GLASS = CLEAN && COUNT && !DYN && std::is_same<J, WfOne>::value;   // glass_direction
+            live = wf_step<CLEAN, ORDER, false, COUNTED_GLASS>(jobs, win, B, slot, R, SH, PX, sec_f(SH, 6), SH.w[7], pc, st,
+                                                               paths, status);
         }
         wf_push(qn, cn, slot, live);
         chunks.advance(pending);
