@@ -1093,6 +1093,7 @@ struct WfRun {
     uint64_t iterations = 0, launches = 0;
     bool drained = false;
     uint32_t drained_slots = 0;
+    const uint32_t* d_drained = nullptr;   // the same on the device, where the host did not poll it
     bool split = false;
 };
 
@@ -1301,10 +1302,13 @@ rtc_status run_wavefront(const DevScene& S, const rtc_render_params* p, const Wf
             }
         }
         // A frame of fewer units than the drain threshold always drains after its second batch (the count of
-        // the first is at most the units): nothing to wait for.
+        // the first is at most the units): nothing to wait for.  That count stays in its counter, which neither
+        // the second batch nor the drain writes.
         if (bounces && units < (int64_t)drain && split_at == 0) {
-            if (b == 0) continue;
-            left = (uint32_t)units;
+            if (b == 0) {
+                run.d_drained = B.ctr + wf_iter(rot).cin;
+                continue;
+            }
             run.drained = true;
             break;
         }
@@ -1351,6 +1355,7 @@ rtc_status launch_wavefront(rtc_context* c, const rtc_scene* s, const rtc_render
     const int64_t units = (int64_t)p->width * p->height * dev_params(p).groups;
     const uint32_t slots = (uint32_t)std::min<int64_t>(units, WF_MAX_SLOTS);
     WfBuffers B;
+    c->d_drained = nullptr;   // the counters start over
     rtc_status r = ensure_wavefront(c, slots, B);
     if (r != RTC_OK) return r;
     RTC_CUDA(after_last_render(c, st));
@@ -1394,6 +1399,7 @@ rtc_status launch_wavefront(rtc_context* c, const rtc_scene* s, const rtc_render
     c->last.iterations = (uint32_t)run.iterations;
     c->last.launches = (uint32_t)run.launches;
     c->last.drained_slots = run.drained_slots;
+    c->d_drained = run.d_drained;
     c->last_timed = true;
     return RTC_OK;
 }
@@ -1431,6 +1437,7 @@ namespace {
 rtc_status launch(rtc_context* c, const rtc_scene* s, const rtc_render_params* p, float4* d_out,
                   unsigned long long* d_counters, cudaStream_t st, uint8_t* d_rgb8) {
     if (p->engine != RTC_ENGINE_MEGAKERNEL) return launch_wavefront(c, s, p, d_out, d_counters, st, d_rgb8);
+    c->d_drained = nullptr;
     c->last = rtc_render_stats{};
     c->last.engine = RTC_ENGINE_MEGAKERNEL;
     c->last.launches = 1;
@@ -1516,9 +1523,16 @@ extern "C" rtc_status rtc_render_device(rtc_context* c, const rtc_scene* s, cons
 extern "C" rtc_status rtc_get_render_stats(rtc_context* c, rtc_render_stats* out) {
     if (!c || !out) return fail(RTC_ERR_INVALID_ARGUMENT, "null argument");
     std::lock_guard<std::mutex> lk(c->mu);
+    if (c->last_timed) RTC_CUDA(cudaEventSynchronize(c->phase_ev[2]));
+    if (c->d_drained) {
+        RtcDeviceScope dev(c->device);
+        RTC_CUDA(dev.error());
+        RTC_CUDA(cudaMemcpyAsync(&c->last.drained_slots, c->d_drained, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+        RTC_CUDA(cudaStreamSynchronize(c->stream));
+        c->d_drained = nullptr;
+    }
     *out = c->last;
     if (c->last_timed) {
-        RTC_CUDA(cudaEventSynchronize(c->phase_ev[2]));
         RTC_CUDA(cudaEventElapsedTime(&out->bulk_ms, c->phase_ev[0], c->phase_ev[1]));
         RTC_CUDA(cudaEventElapsedTime(&out->drain_ms, c->phase_ev[1], c->phase_ev[2]));
         out->extend_launches = c->kev_ext;

@@ -160,6 +160,7 @@ extern "C" rtc_status rtc_render_batch(rtc_context* c, const rtc_job* jobs, uint
     }
     if (!E.all_done()) return rtc_set_error(RTC_ERR_DEVICE_CHECK, "batch ended with unfinished images");
     c->last = rtc_render_stats{};
+    c->d_drained = nullptr;
     c->last.engine = RTC_ENGINE_WAVEFRONT;
     c->last.iterations = (uint32_t)E.iterations();
     c->last.launches = (uint32_t)E.launches();

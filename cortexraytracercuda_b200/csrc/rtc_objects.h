@@ -40,6 +40,7 @@ struct rtc_context {
     cudaEvent_t split_ev[2] = {nullptr, nullptr};
     rtc_render_stats last{};
     bool last_timed = false;
+    const uint32_t* d_drained = nullptr;   // where `last.drained_slots` is still on the device
     std::vector<cudaEvent_t> kev;      // per-launch timing events (RTC_FLAG_KERNEL_TIMING)
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> kev_pairs;   // extend pairs, then shade pairs
     uint32_t kev_ext = 0, kev_shade = 0;   // pairs used by the last render

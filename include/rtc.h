@@ -453,8 +453,7 @@ rtc_status rtc_render_device(rtc_context* ctx, const rtc_scene* scene, const rtc
                              void* stream);
 
 /* Statistics of the last render on this context (wavefront engine): iterations of (extend, shade),
- * kernel launches, whether the drain kernel ran and for how many slots (at most, where the frame was
- * queued without a poll), and the device time of the
+ * kernel launches, whether the drain kernel ran and for how many slots, and the device time of the
  * bulk iterations and of the drain kernel (ms, from CUDA events; the call waits for the render). */
 typedef struct rtc_render_stats {
     uint32_t iterations;
