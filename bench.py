@@ -920,7 +920,7 @@ def main():
     clk = clocks.stop()
     launches_per_step = int(ctx.last_stats()["launches"])
     # the per-kernel split, from two more frames with CUDA events around every extend and shade launch
-    # (untimed: those events cost ~5 ms of a ~75 ms frame)
+    # (untimed: they also keep the split kernels to the drain and take ~56 ms, the frames above ~49)
     kstats = []
     if wavefront:
         params.flags |= FLAG_KERNEL_TIMING
@@ -971,6 +971,8 @@ def main():
                 "alg_bytes_per_launch": int(ext_bytes / max(ext_launches, 1)),
                 "avg_launch_ms": round(ext_ms / max(ext_launches, 1), 4), "kernel_ms_per_frame": round(ext_ms, 3),
                 "share_of_frame": round(ext_ms / float(np.mean([st["bulk_ms"] + st["drain_ms"] for st in kstats])), 3),
+                "split_frames": "two frames apart from the timed ones, an event pair around every launch: extend and shade "
+                                "kernels to the drain, where the timed frames run their later iterations in wf_bounces",
                 "per_frame": {"rays": ext_rays, "node_visits": ext_nodes, "prim_tests": ext_prims},
                 "bytes_per_ray": round(ext_bytes / max(ext_rays, 1), 1),
                 "frame": {"shade_ms": round(float(np.mean([st["shade_ms"] for st in kstats])), 3),
