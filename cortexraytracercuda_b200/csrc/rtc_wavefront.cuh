@@ -82,7 +82,8 @@ __device__ __forceinline__ uint32_t* wf_sec(const WfBuffers& B, uint32_t slot, i
     return sec == SEC_PIXEL ? B.px + 8 * (size_t)slot : B.rec + WF_REC_WORDS * (size_t)slot + 8 * sec;
 }
 
-// OWN: through L1, for a sector that this thread itself wrote in this kernel (wf_bounces).
+// OWN: through L1, for a sector that earlier kernels wrote (L1 holds nothing of theirs when a kernel starts) or
+// this thread itself in this one (wf_bounces), and that no other thread touches meanwhile.
 template <bool OWN = false>
 __device__ __forceinline__ Sec ld_sec(const uint32_t* p) {
     Sec s;
@@ -720,8 +721,9 @@ __global__ void RTC_SHADE_BOUNDS wf_shade_ring(WfTable jobs, WfBuffers B, WfIter
 // bounces, so a batch of iterations over a queue that no longer fills the GPU costs one launch instead of
 // two a bounce, each with its ramp and its tail; over a long queue the split kernels win (64 registers
 // against this one's 96, and no lanes that wait for other lanes' materials).  A step goes through the slot's
-// record exactly as the split kernels' does - the same arithmetic in the same order - so where a bounce runs
-// does not change it.  Rule (run_wavefront): at most 2,048 queued slots per SM.  Measured at 1,024 / 2,048 /
+// record exactly as the split kernels' does, the same arithmetic in the same order.  In the FMA flavours the
+// compiler rounds it as in the fixed-stride shade kernel (compared bit for bit, tests/test_gpu_drain.py), not as
+// in the counter-fed one, whose frames stay with the split kernels.  Rule (run_wavefront): at most 2,048 queued slots per SM.  Measured at 1,024 / 2,048 /
 // 4,096 slots per SM against the split kernels only: spheres 1280x720 55.5 / 54.9 / 55.2 against 56.8 ms,
 // meshes (1.31 M triangles) 62.9 / 62.3 / 62.3 against 64.1, transforms 333x251 7.00 / 6.90 / 6.91 against
 // 7.24; Cornell 256x256 1.60 against 1.79, 64x48 preview 0.26 against 0.44 ms.  96 registers (20 warps per

@@ -610,7 +610,8 @@ rtc_status rtc_server_get_stats(rtc_server* server, rtc_server_stats* stats);
 /* Closest-hit queries on arbitrary rays (hit-identity tests).  rays: n x 8 floats
  * (ox, oy, oz, tmin, dx, dy, dz, tmax) in host memory; `depth`/`max_depth` decide light visibility as
  * in the reference's world.hit (directional_light.cuh:106).  Outputs (host, n each, may be NULL):
- * prim_id (-1 on a miss) and t. */
+ * prim_id (-1 on a miss) and t.  The context keeps the call's device block, up to 64 MiB (1.6 M rays), for the
+ * next call until it is destroyed; larger blocks are freed when the call returns. */
 rtc_status rtc_trace_closest(rtc_context* ctx, const rtc_scene* scene, const float* rays, uint32_t n,
                              int32_t depth, int32_t max_depth, int32_t* prim_id, float* t);
 /* rtc_trace_closest with render flags: RTC_FLAG_WIDE_BVH walks the 8-wide nodes (where the scene has
