@@ -188,18 +188,21 @@ struct PathCounters {
     uint32_t rays, nodes, prims;
 };
 
-// A dielectric's dot(n, d) and its scattered direction, reflect or refract (rtc_math.cuh).  The FMA flavours'
-// compiler rounds that dot product in one of several ways, by the kernel around it.  COUNTED writes out the way
-// of clean mode's instrumented shade kernel of one image, so that its images do not move with that kernel's code.
-__device__ __forceinline__ float glass_dot(V3 n, V3 d) {
-    return __fadd_rn(__fmaf_rn(n.x, d.x, __fmul_rn(n.y, d.y)), __fmul_rn(n.z, d.z));
+// A dielectric's incidence cosine and its scattered direction, reflect or refract (rtc_math.cuh).  The FMA
+// flavours' compiler rounds their dot(n, d) in one of several ways, by the kernel around it.  COUNTED writes out
+// the ways of clean mode's instrumented shade kernel of one image, so that its images do not move with that
+// kernel's code.
+template <bool COUNTED>
+__device__ __forceinline__ float glass_cosine(V3 d, V3 n) {
+    if constexpr (!COUNTED) return dot(neg(d), n);
+    else return -__fadd_rn(__fmaf_rn(n.y, d.y, __fmul_rn(n.x, d.x)), __fmul_rn(n.z, d.z));
 }
 template <bool COUNTED>
 __device__ __forceinline__ V3 glass_direction(V3 d, V3 n, bool reflected, float eta) {
     if constexpr (!COUNTED) {
         return reflected ? reflect(d, n) : refract(d, n, eta);
     } else {
-        const float dn = glass_dot(n, d);
+        const float dn = __fadd_rn(__fmaf_rn(n.x, d.x, __fmul_rn(n.y, d.y)), __fmul_rn(n.z, d.z));
         if (reflected) return sub(d, mul(mul(n, dn), 2.0f));
         const float k = __fmaf_rn(-__fmul_rn(eta, eta), __fmaf_rn(-dn, dn, 1.0f), 1.0f);
         if (!(k >= 0.0f)) return v3(0.0f, 0.0f, 0.0f);
@@ -231,7 +234,7 @@ __device__ __forceinline__ void scatter_bounce(const DevScene& S, Ray& r, Hit& h
         // dielectric::scatter (dielectric.cuh:32-52) with Schlick (dielectric.cuh:57-63)
         float ratio = h.front ? (1.0f / mf.y) : mf.y;
         V3 ud = unit(r.d);
-        float ct = COUNTED_GLASS ? -glass_dot(h.n, ud) : dot(neg(ud), h.n);
+        float ct = glass_cosine<COUNTED_GLASS>(ud, h.n);
         float cos_theta = ct < 1.0f ? ct : 1.0f;
         float sin_theta = sqrtf(1.0f - cos_theta * cos_theta);
         bool cannot_refract = ratio * sin_theta > 1.0f;

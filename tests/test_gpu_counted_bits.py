@@ -31,3 +31,18 @@ def test_counted_glass_pixels(ctx):
     words = out.cpu().numpy().view(np.uint32)
     for at, want in PIXELS.items():
         assert tuple(int(w) for w in words[at][:3]) == want
+
+
+def test_counted_glass_decision_pixel(ctx):
+    """A refraction whose choice against reflection hangs on the incidence cosine's last bit."""
+    import torch
+    s = configs.SCENES["xforms"][0]()
+    s.camera.aspect = W / H
+    ds = DeviceScene(ctx, s)
+    p = RenderParams(width=W, height=H, spp=64, max_depth=10, mode=MODE_CLEAN, seed=82, engine=ENGINE_WAVEFRONT)
+    out = torch.empty(H, W, 4, device="cuda")
+    cnt = torch.zeros(8, dtype=torch.int64, device="cuda")
+    ds.render_device(p, out.data_ptr(), None, cnt.data_ptr())
+    torch.cuda.synchronize()
+    words = out.cpu().numpy().view(np.uint32)
+    assert tuple(int(w) for w in words[569, 1336][:3]) == (0x41691b6c, 0x3f84cf46, 0x3f816c83)
