@@ -67,7 +67,7 @@ SOURCES = [
     ("bvh_build.cpp", "bvh_build", "cxx", []),
 ]
 HEADERS = ["rtc_dev.h", "rtc_math.cuh", "rtc_trace.cuh", "rtc_path.cuh", "rtc_wavefront.cuh", "rtc_kernels.h",
-           "bvh_build.h", "rtc_internal.h", "rtc_objects.h", "rtc_engine.h", "rtc_claims.h"]
+           "bvh_build.h", "rtc_internal.h", "rtc_objects.h", "rtc_engine.h"]
 
 
 def _newer(target: Path, deps) -> bool:

@@ -77,8 +77,8 @@ rtc_status Engine::reset() {
     ENG_CUDA(cudaStreamSynchronize(st_));
     std::fill(ring_.begin(), ring_.end(), EngineJob{});
     lo_ = hi_ = staged_from_ = 0;
-    claims_ = RingClaims{};
-    next_ = 0;
+    limit_ = next_ = 0;
+    live_ = 0;
     status_ = 0;
     observed_ = false;
     refill_ = false;
@@ -99,8 +99,8 @@ rtc_status Engine::admit(DevJob job, uint64_t tag, uint64_t* seq) {
     const uint64_t s = hi_++;
     const uint32_t slot = (uint32_t)(s & (cfg_.ring - 1));
     const uint64_t npix = (uint64_t)job.P.num_pixels;
-    job.begin = claims_.limit;
-    claims_.limit += npix * (uint64_t)std::max(1, job.P.groups);   // work units: pixel x sample group
+    job.begin = limit_;
+    limit_ += npix * (uint64_t)std::max(1, job.P.groups);   // work units: pixel x sample group
     h_jobs_[slot] = job;
     ENG_CUDA(cudaMemcpyAsync(d_jobs_ + slot, h_jobs_ + slot, sizeof(DevJob), cudaMemcpyHostToDevice, st_));
     uint32_t* d_done = (uint32_t*)(d_prog_ + sizeof(WfFeed));
@@ -123,7 +123,7 @@ rtc_status Engine::enqueue_admit() {
     WfTableArgs A{d_jobs_, (WfFeed*)d_prog_, (uint32_t*)(d_prog_ + sizeof(WfFeed)), cfg_.ring - 1};
     WfLaunch L{};
     L.w = wf_iter(it_);
-    L.win.limit = claims_.limit;
+    L.win.limit = limit_;
     L.win.lo = (uint32_t)lo_;
     L.win.hi = (uint32_t)hi_;
     L.status = d_status_;
@@ -146,7 +146,6 @@ rtc_status Engine::enqueue_poll() {
                              cudaMemcpyDeviceToHost, st_));
     ENG_CUDA(cudaEventRecord(poll_ev_[slot], st_));
     poll_batch_[slot] = batch_no_;
-    claims_.polled(slot);
     return RTC_OK;
 }
 
@@ -159,7 +158,7 @@ rtc_status Engine::observe(int slot) {
     std::memcpy(&status_, h + POLL_STATUS, sizeof status_);
     std::memcpy(&feed, h + POLL_FEED, sizeof feed);
     const uint32_t* done = (const uint32_t*)(h + POLL_DONE);
-    claims_.observe(slot, feed.next, live);
+    live_ = live;
     next_ = feed.next;
     for (uint64_t s = lo_; s < hi_; ++s) {
         EngineJob& J = ring_[s & (cfg_.ring - 1)];
@@ -174,7 +173,7 @@ rtc_status Engine::observe(int slot) {
     while (lo_ < hi_ && ring_[lo_ & (cfg_.ring - 1)].done) ++lo_;
     observed_ = true;
     // no live slot while work is unfinished: idle slots must claim the remaining pixels
-    if (live == 0 && jobs_done_ < jobs_total_) refill_ = true;
+    if (live_ == 0 && jobs_done_ < jobs_total_) refill_ = true;
     return RTC_OK;
 }
 
@@ -198,7 +197,7 @@ rtc_status Engine::enqueue_iterations() {
     // balances without atomics (16 images of 320x240, 900 K pixels: 23.3 against 25.9 ms).  The shade kernel
     // keeps the counter (striding, one and four waves: within 2% and up to 5% slower).
     const int wave = cfg_.num_sms * 8 * 128 / cfg_.block;   // 1,024 threads per SM
-    const bool down = claims_.runs_down(cfg_.slots);
+    const bool down = runs_down();
     auto launch_pair = [&](uint64_t k) {
         L.w = wf_iter(k);
         L.dynamic = rtc_dynamic_chunks(!down);

@@ -14,11 +14,11 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <vector>
 
 #include "../../include/rtc.h"
-#include "rtc_claims.h"
 #include "rtc_dev.h"
 #include "rtc_kernels.h"
 
@@ -75,8 +75,8 @@ public:
 
     // host view (as of the last observed poll)
     bool all_done() const { return jobs_done_ == jobs_total_; }
-    bool all_claimed() const { return observed_ && next_ >= claims_.limit; }
-    uint32_t live() const { return claims_.live; }
+    bool all_claimed() const { return observed_ && next_ >= limit_; }
+    uint32_t live() const { return live_; }
     uint64_t in_flight() const { return jobs_total_ - jobs_done_; }
     uint32_t observed_status() const { return status_; }   // kernel status word as of the last poll
     size_t device_bytes() const { return device_bytes_; }
@@ -101,6 +101,12 @@ private:
     rtc_status observe(int slot);
     rtc_status enqueue_iterations();
     void drop_graph();
+    // Whether every unit not yet claimed has an idle slot waiting for it, by what was last observed (late, so
+    // on the safe side): from here on the queue only runs down.
+    bool runs_down() const {
+        const uint64_t unclaimed = limit_ - std::min(next_, limit_);
+        return unclaimed + live_ <= cfg_.slots;
+    }
 
     EngineConfig cfg_;
     cudaStream_t st_ = nullptr;
@@ -124,8 +130,9 @@ private:
     std::vector<EngineJob> ring_;
     uint64_t lo_ = 0, hi_ = 0;      // jobs [lo_, hi_) are admitted and not yet observed done (lo_ oldest)
     uint64_t staged_from_ = 0;      // jobs [staged_from_, hi_) are staged, not yet published
-    RingClaims claims_;             // units admitted, claimed and live
+    uint64_t limit_ = 0;            // pixels admitted (global sequence)
     uint64_t next_ = 0;             // observed claim cursor
+    uint32_t live_ = 0;             // observed live slots
     uint32_t status_ = 0;           // observed kernel status word
     size_t device_bytes_ = 0;
     bool observed_ = false;
